@@ -241,7 +241,7 @@ struct gs_ctx {
   int com_mode = kComF32;
   int sort_items = kSortItems;     // tuning: keys per thread of a sort tile (0: by galaxy size; 4, 8 or 16)
   int sort_eff = kSortItems;       // the layout's keys per thread (sort_items, or chosen by size)
-  int walk_bps = kWalkBlocksPerSM; // tuning: persistent walk blocks per SM (1..8; < 8: 72-register build)
+  int walk_bps = kWalkBlocksPerSM; // tuning: persistent walk blocks per SM (1..8; at most kWalkResident run)
   int walk_group = 32;             // tuning: walk group size (0: by galaxy size; 4, 8, 16 or 32 particles)
   int walk_split = 1;              // tuning: walk splits per work item of a lone galaxy (0: by its size; 1, 2, 4, 8)
   uint32_t walk_items[4] = {0, 0, 0, 0};  // work items per lanes-per-particle class (1, 2, 4, 8)
@@ -563,7 +563,8 @@ int ensure_layout(gs_ctx* c) {
   c->seg_host = h;
   c->sort_eff = items_eff;
   const uint32_t most = std::max(std::max(items[0], items[1]), std::max(items[2], items[3]));
-  c->walk_grid = std::min<uint32_t>(std::max<uint32_t>(1, cdiv(most, kWalkWarps)), (uint32_t)c->sms * c->walk_bps);
+  c->walk_grid = std::min<uint32_t>(std::max<uint32_t>(1, cdiv(most, kWalkWarps)),
+                                    (uint32_t)c->sms * std::min(c->walk_bps, kWalkResident));
   for (int k = 0; k < 4; k++) c->walk_items[k] = items[k];
   c->drop_graphs();
   c->lay_dirty = false;
@@ -635,11 +636,11 @@ void enqueue_build(gs_ctx* c, const float4* pos, uint32_t stride, int com_mode, 
     launch_pdl(tree_leaves_kernel<kComF32>, L.flag_tiles, kLeafThreads, s, b, L, pos, stride, c->st);
 }
 
-template <int MINB, int LPP>
+template <int LPP>
 void launch_walk(int v, uint32_t g, cudaStream_t s, const WalkArgs& a) {
   switch (v) {
 #define GS_WALK_CASE(V, SF, DBG, ONE, COMP) \
-  case V: launch_pdl(walk_kernel<SF, DBG, ONE, COMP, MINB, LPP>, g, kWalkThreads, s, a); break;
+  case V: launch_pdl(walk_kernel<SF, DBG, ONE, COMP, LPP>, g, kWalkThreads, s, a); break;
     GS_WALK_CASE(0, false, false, false, false)
     GS_WALK_CASE(1, true, false, false, false)
     GS_WALK_CASE(2, false, true, false, false)
@@ -686,16 +687,14 @@ void enqueue_walk(gs_ctx* c, int sf) {
   a.split_arrive = c->split_arrive;
   a.split_stride = one ? a.seg0.n : 0u;
   const int v = (sf ? 1 : 0) | (c->debug ? 2 : 0) | (one ? 4 : 0) | (c->walk_comp ? 8 : 0);
-  // one launch per walk group size present (a single galaxy: its own); 8 blocks
-  // per SM: the 64-register build, fewer: the 72-register build (groups of 32)
+  // one launch per walk group size present (a single galaxy: its own)
   for (int k = 0; k < 4; k++) {
     if (!c->walk_items[k]) continue;
     const uint32_t gk = std::min<uint32_t>(g, std::max<uint32_t>(1, cdiv(c->walk_items[k], kWalkWarps)));
-    if (k == 1) launch_walk<kWalkBlocksPerSM, 2>(v, gk, s, a);
-    else if (k == 2) launch_walk<kWalkBlocksPerSM, 4>(v, gk, s, a);
-    else if (k == 3) launch_walk<kWalkBlocksPerSM, 8>(v, gk, s, a);
-    else if (c->walk_bps >= kWalkBlocksPerSM) launch_walk<kWalkBlocksPerSM, 1>(v, gk, s, a);
-    else launch_walk<kWalkBlocksWide, 1>(v, gk, s, a);
+    if (k == 0) launch_walk<1>(v, gk, s, a);
+    else if (k == 1) launch_walk<2>(v, gk, s, a);
+    else if (k == 2) launch_walk<4>(v, gk, s, a);
+    else launch_walk<8>(v, gk, s, a);
   }
   // per-galaxy FP64 diagnostics of this walk
   launch_pdl(diag_reduce_kernel, c->lay.diag_chunks, 32 * kPartials, s, (const double*)c->partials, c->lay,
@@ -1054,7 +1053,7 @@ int gs_create_on(int device, uint32_t N, const float* particles8, const float* s
   }
   c->palloc.init(0);
   c->single = true;
-  c->walk_bps = kWalkBlocksWide;  // one galaxy: the 72-register walk measured faster
+  c->walk_bps = kWalkResident;
   c->walk_group = 0;              // one galaxy: walk groups by its size (a pool fills the GPU with 32s)
   c->walk_split = 0;              // and walk splits by its size
   c->sort_items = 0;              // and sort tiles by its size

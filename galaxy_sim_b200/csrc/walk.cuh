@@ -16,19 +16,18 @@
 //     ranges and stages their children into shared memory by one coalesced load
 //     (one child per lane, structure of arrays), so the round's stack, ballot and
 //     staging work is shared by up to 32 children.
-//   * Children are tested two at a time, and an opened leaf's particles are
-//     staged the same way and summed two at a time, with sm_100's packed
-//     FP32x2 FMA/ADD/MUL; accumulation is predicated, not branched (a child or
-//     source a lane does not take gets r^2 + eps^2 = +inf, so rsqrt gives 0).
-//     Walk groups of 16 or fewer stage a round's opened leaves back to back and
-//     sum them in batches of 32 source pairs (see the leaf section).
+//   * Children are tested two at a time with sm_100's packed FP32x2 FMA/ADD/MUL;
+//     accumulation is predicated, not branched (a child a lane does not take gets
+//     r^2 + eps^2 = +inf, so rsqrt gives 0).
+//   * Opened leaves are queued and summed in windows of up to 96 source pairs, by
+//     subgroups of 8 particles with 4 lanes each (leaf_flush).
 //   * Warps are persistent and take work items from an atomic counter (load
 //     balance across the dense core); per-item FP64 partials of the
 //     diagnostics replace a block-wide barrier.
 //   * Walk group size: a work item is 32, 16, 8 or 4 Morton-consecutive
 //     particles (LPP = 1, 2, 4 or 8 lanes per particle). With LPP > 1 the lanes of a
-//     particle split the round's slot pairs and each opened leaf's source pairs
-//     between them and add their partial sums by shuffles at the end, so a
+//     particle split the round's slot pairs between them (items of 8 or 4 also the
+//     leaf pairs) and add their partial sums by shuffles at the end, so a
 //     small galaxy keeps more warps busy and each warp walks the union of
 //     fewer frontiers. A 32-particle walk group (layout, diagnostics) holds LPP
 //     items. The split changes the order of the force sums, so results change
@@ -58,10 +57,13 @@ constexpr int kWalkRanges = GS_WALK_RANGES;  // child ranges popped and tested p
 static_assert(kWalkRanges >= 1 && kWalkRanges <= 4, "a round stages at most one child per lane");
 // ranges; a round explores kWalkRanges paths, each leaving <= 7 pending ranges per depth
 constexpr int kWalkStack = 8 * 11 * kWalkRanges;
-// The walk is compiled twice: for 8 resident blocks per SM (64 registers per
-// thread) and for 7 (72 registers, fewer spills); the launch tuning picks one.
+// Resident blocks per SM the walk is compiled for: 72 registers per thread without
+// spills, and 31.5 KB of staging per block, of which 7 fit an SM. The launch tuning
+// accepts 1..8; more than the resident blocks launch no further ones. (Before leaf
+// sums were queued, a second build of 64 registers for 8 blocks ran the 96-galaxy
+// pool in 7.569 ms against 7.572 ms for this one.)
 constexpr int kWalkBlocksPerSM = 8;
-constexpr int kWalkBlocksWide = 7;
+constexpr int kWalkResident = 7;
 constexpr uint32_t kWalkGroup = 32;             // particles per walk group (layout, diagnostics)
 constexpr uint32_t kWalkParts = 8;              // partial-sum slots per walk group (the largest LPP)
 // with the walk group chosen by size, galaxies of at most this many particles
@@ -156,30 +158,43 @@ struct WalkArgs {
   uint32_t split_stride;
 };
 
+// Opened leaves wait in a per-warp queue until they hold kLeafFlush source pairs
+// (or the walk ends); their direct sums then run over windows of up to
+// kLeafWindow staged pairs (see leaf_flush).
+#ifndef GS_LEAF_WINDOW
+#define GS_LEAF_WINDOW 96
+#endif
+#ifndef GS_LEAF_FLUSH
+#define GS_LEAF_FLUSH 72
+#endif
+constexpr int kLeafWindow = GS_LEAF_WINDOW;
+constexpr int kLeafFlush = GS_LEAF_FLUSH;
+constexpr uint32_t kLeafMax = 16;  // particles of a queued leaf (larger ones are summed at once)
+static_assert(kLeafWindow % 32 == 0 && kLeafWindow <= 128, "a lane stages whole pairs; 7-bit pair indices");
+// a queue entry packs the first particle and the count: particle indices have 27 bits
+constexpr int kLeafCountShift = 27;
+
 // Per-warp shared staging.
 struct WalkSmem {
   uint2 stack[kWalkStack];          // {first child | (count-1) << 29, lane mask}
-  // staged child ranges, pair-interleaved so a packed test reads two 128-bit
-  // words: cxy[4p..4p+3] = {x(2p), x(2p+1), y(2p), y(2p+1)}, czm likewise {z, m}
-  __align__(16) float cxy[16 * kWalkRanges];
-  __align__(16) float czm[16 * kWalkRanges];
-  float cs2[8 * kWalkRanges];
-  uint32_t cnode[8 * kWalkRanges];  // node index of each staged child
-  uint4 cmeta[8 * kWalkRanges];     // {child, info, own-leaf size bits, massive}
-  // staged leaf sources, pair-interleaved the same way (pairs 0..32)
-  __align__(16) float lxy[136];
-  __align__(16) float lzm[136];
-  uint4 bl[32];  // a round's opened leaves: {first particle, count, opening mask, first pair}
+  uint2 q[kLeafFlush + 32];         // opened leaves: {first | (count-1) << 27, opening mask}
+  union {
+    struct {
+      // staged child ranges, pair-interleaved so a packed test reads two 128-bit
+      // words: cxy[4p..4p+3] = {x(2p), x(2p+1), y(2p), y(2p+1)}, czm likewise {z, m}
+      __align__(16) float cxy[16 * kWalkRanges];
+      __align__(16) float czm[16 * kWalkRanges];
+      float cs2[8 * kWalkRanges];
+    };
+    uint2 pinfo[kLeafWindow];       // a window's source pairs: {first source | both << 31, opening mask}
+  };
+  // staged leaf sources, pair-interleaved the same way
+  __align__(16) float lxy[4 * kLeafWindow];
+  __align__(16) float lzm[4 * kLeafWindow];
+  // the window's pairs of one subgroup: byte offset of the pair in lxy | opening mask << 24
+  uint32_t list[kLeafWindow + 4];
 };
 
-// Direct sum of a staged leaf segment [off, off + k) for the lanes in `me`
-// (nbody_bh.wgsl:117-131), used by walk groups of 32: two sources per packed
-// step, up to kmax >= k (staged sources past a leaf's count are massless zeros).
-// A particle served by LPP lanes splits the source pairs: lane `sub` takes pairs
-// sub, sub + LPP, ... With soft (eps^2 a normal float) the self pair is included (zero
-// force at r = 0) and its potential removed once at the end of the walk via
-// selfw (counted by the lane whose share holds it); otherwise it is skipped per
-// pair.
 // Reciprocal square root for the walk's r^2 + eps^2, which is never subnormal
 // (eps^2 is zero or at least the smallest normal float, and zero softening adds
 // that smallest normal instead): the flush-to-zero form gives the same result as
@@ -190,103 +205,201 @@ __device__ __forceinline__ float rsqrt_walk(float x) {
   return r;
 }
 
-template <int LPP, typename Smem>
-__device__ __forceinline__ void leaf_sum(const Smem& S, uint32_t off, uint32_t k, uint32_t kmax, uint32_t jself,
-                                         bool me, bool soft, float2 px, float2 py, float2 pz,
-                                         float eps2, float2& ax, float2& ay, float2& az,
-                                         float2& pt, float& selfw, unsigned long long& npair,
-                                         bool dbg, uint32_t sub) {
-  if (soft) {
-    // a lane that did not open the leaf gets eps^2 = +inf: its r^2 + eps^2 is
-    // +inf, rsqrt gives 0 and every term of the pair vanishes (r is finite)
-    const float e2me = me ? eps2 : INFINITY;
-    if (me && jself < k && ((jself >> 1) % LPP) == sub) selfw += 1.0f;
-    for (uint32_t j = 2 * sub; j < kmax; j += 2 * LPP) {
-      const float4 jxy = *reinterpret_cast<const float4*>(&S.lxy[2 * (off + j)]);
-      const float4 jzm = *reinterpret_cast<const float4*>(&S.lzm[2 * (off + j)]);
-      const float2 jx = make_float2(jxy.x, jxy.y), jy = make_float2(jxy.z, jxy.w);
-      const float2 jz = make_float2(jzm.x, jzm.y), jm = make_float2(jzm.z, jzm.w);
-      const float2 ex = __fadd2_rn(jx, px), ey = __fadd2_rn(jy, py), ez = __fadd2_rn(jz, pz);
-      const float2 e2 = __ffma2_rn(ex, ex, __ffma2_rn(ey, ey, __ffma2_rn(ez, ez, make_float2(e2me, e2me))));
-      const float2 ri = make_float2(rsqrt_walk(e2.x), rsqrt_walk(e2.y));
-      const float2 mr = __fmul2_rn(jm, ri);
-      const float2 ff = __fmul2_rn(__fmul2_rn(mr, ri), ri);
-      ax = __ffma2_rn(ex, ff, ax);
-      ay = __ffma2_rn(ey, ff, ay);
-      az = __ffma2_rn(ez, ff, az);
-      pt = __fadd2_rn(pt, mr);
-      if (dbg && me) npair += (j < k && j != jself) + (j + 1 < k && j + 1 != jself);
-    }
-  } else {
-    for (uint32_t j = 2 * sub; j < kmax; j += 2 * LPP) {
-      const float4 jxy = *reinterpret_cast<const float4*>(&S.lxy[2 * (off + j)]);
-      const float4 jzm = *reinterpret_cast<const float4*>(&S.lzm[2 * (off + j)]);
-      const float2 jx = make_float2(jxy.x, jxy.y), jy = make_float2(jxy.z, jxy.w);
-      const float2 jz = make_float2(jzm.x, jzm.y), jm = make_float2(jzm.z, jzm.w);
-      const float2 ex = __fadd2_rn(jx, px), ey = __fadd2_rn(jy, py), ez = __fadd2_rn(jz, pz);
-      const float2 e2 = __ffma2_rn(ex, ex, __ffma2_rn(ey, ey, __ffma2_rn(ez, ez, make_float2(eps2, eps2))));
-      const bool u0 = me && j < k && j != jself;
-      const bool u1 = me && j + 1 < k && j + 1 != jself;
-      const float2 ri = make_float2(u0 ? rsqrt_walk(e2.x) : 0.0f, u1 ? rsqrt_walk(e2.y) : 0.0f);
-      const float2 mr = __fmul2_rn(jm, ri);
-      const float2 ff = __fmul2_rn(__fmul2_rn(mr, ri), ri);
-      ax = __ffma2_rn(ex, ff, ax);
-      ay = __ffma2_rn(ey, ff, ay);
-      az = __ffma2_rn(ez, ff, az);
-      pt = __fadd2_rn(pt, mr);
-      if (dbg) npair += u0 + u1;
-    }
-  }
-}
-
-// Direct sums of one staged batch of leaf sources for walk groups of 16 or fewer
-// (nbody_bh.wgsl:117-131): up to 32 source pairs, pair t pair-interleaved at
-// lxy/lzm[4t..4t+3], each pair from one leaf (a leaf of odd count ends in a
-// massless zero). A particle served by LPP lanes splits the pairs: lane `sub`
-// takes pairs sub, sub + LPP, ... Bit LPP * kk of `pm` tells whether the
-// particle opened the leaf of pair sub + LPP * kk.
-// With soft (eps^2 a normal float) a pair the lane does not take gets eps^2 = +inf: r^2 +
-// eps^2 is then +inf, rsqrt gives 0 and every term vanishes (r is finite); the
-// self pair is included (zero force at r = 0) and its potential removed once at
-// the end of the walk. Without softening the self pair (batch source `selfloc`)
-// is skipped per pair. Pairs past nbp hold massless zeros and are never in pm.
-template <int LPP, bool SOFT, typename Smem>
-__device__ __forceinline__ void leaf_batch(const Smem& S, uint32_t nbp, uint32_t pm, uint32_t selfloc,
-                                           float2 px, float2 py, float2 pz, float eps2, float2& ax,
-                                           float2& ay, float2& az, float2& pt, uint32_t sub) {
-  constexpr int NB = 32 / LPP;  // steps of a lane over a full batch
-  const float* lx = &S.lxy[4 * sub];
-  const float* lz = &S.lzm[4 * sub];
-#pragma unroll
-  for (int kk = 0; kk < NB; kk++) {
-    if ((kk * LPP) % 4 == 0 && kk * LPP >= (int)nbp) break;  // one check per four pairs
-    const float4 jxy = *reinterpret_cast<const float4*>(lx + 4 * LPP * kk);
-    const float4 jzm = *reinterpret_cast<const float4*>(lz + 4 * LPP * kk);
-    const float2 jx = make_float2(jxy.x, jxy.y), jy = make_float2(jxy.z, jxy.w);
-    const float2 jz = make_float2(jzm.x, jzm.y), jm = make_float2(jzm.z, jzm.w);
-    const float2 ex = __fadd2_rn(jx, px), ey = __fadd2_rn(jy, py), ez = __fadd2_rn(jz, pz);
-    const bool me = (pm >> (LPP * kk)) & 1u;
-    float2 ri;
-    if (SOFT) {
-      const float e2me = me ? eps2 : INFINITY;
-      const float2 e2 = __ffma2_rn(ex, ex, __ffma2_rn(ey, ey, __ffma2_rn(ez, ez, make_float2(e2me, e2me))));
-      ri = make_float2(rsqrt_walk(e2.x), rsqrt_walk(e2.y));
-    } else {
-      const uint32_t j2 = 2 * (sub + LPP * kk);  // the pair's first source in the batch
-      const float2 e2 = __ffma2_rn(ex, ex, __ffma2_rn(ey, ey, __ffma2_rn(ez, ez, make_float2(eps2, eps2))));
-      ri = make_float2(me && j2 != selfloc ? rsqrt_walk(e2.x) : 0.0f,
-                       me && j2 + 1 != selfloc ? rsqrt_walk(e2.y) : 0.0f);
-    }
-    const float2 mr = __fmul2_rn(jm, ri);
-    const float2 ff = __fmul2_rn(__fmul2_rn(mr, ri), ri);
-    ax = __ffma2_rn(ex, ff, ax);
-    ay = __ffma2_rn(ey, ff, ay);
-    az = __ffma2_rn(ez, ff, az);
-    pt = __fadd2_rn(pt, mr);
-  }
-}
-
 __device__ inline float2 f2(float a) { return make_float2(a, a); }
+
+// Packed sums of a particle: acceleration / G and sum of m / r.
+struct Sums {
+  float2 ax, ay, az, pt;
+};
+
+// One packed step of a direct sum (nbody_bh.wgsl:117-131): the two staged sources
+// of the pair whose {x, x, y, y} lie `at` bytes into lxy against the particle at -p,
+// with e0 and e1 the softening each source gets (+inf: r^2 + eps^2 is +inf, rsqrt
+// gives 0 and every term vanishes, as r is finite).
+template <typename Smem>
+__device__ __forceinline__ void pair_step(const Smem& S, uint32_t at, float2 px, float2 py, float2 pz, float e0, float e1, Sums& s) {
+  const float4 jxy = *reinterpret_cast<const float4*>(reinterpret_cast<const char*>(S.lxy) + at);
+  const float4 jzm = *reinterpret_cast<const float4*>(reinterpret_cast<const char*>(S.lzm) + at);
+  const float2 jx = make_float2(jxy.x, jxy.y), jy = make_float2(jxy.z, jxy.w);
+  const float2 jz = make_float2(jzm.x, jzm.y), jm = make_float2(jzm.z, jzm.w);
+  const float2 ex = __fadd2_rn(jx, px), ey = __fadd2_rn(jy, py), ez = __fadd2_rn(jz, pz);
+  // the softening enters through two scalar FMAs: no register pair to fill for it
+  const float2 e2 = __ffma2_rn(ex, ex, __ffma2_rn(ey, ey, make_float2(fmaf(ez.x, ez.x, e0), fmaf(ez.y, ez.y, e1))));
+  const float2 ri = make_float2(rsqrt_walk(e2.x), rsqrt_walk(e2.y));
+  const float2 mr = __fmul2_rn(jm, ri);
+  const float2 ff = __fmul2_rn(__fmul2_rn(mr, ri), ri);
+  s.ax = __ffma2_rn(ex, ff, s.ax);
+  s.ay = __ffma2_rn(ey, ff, s.ay);
+  s.az = __ffma2_rn(ez, ff, s.az);
+  s.pt = __fadd2_rn(s.pt, mr);
+}
+
+// Direct sum of one staged chunk of k sources of a leaf of more than kLeafMax
+// particles, for the lanes in `me`. A particle served by LPP lanes splits the
+// source pairs: lane `sub` takes pairs sub, sub + LPP, ... With soft (eps^2 a normal
+// float) the self pair is included (zero force at r = 0; its potential is removed
+// once at the end of the walk); otherwise the particle's own source jself is skipped.
+// A source past k is staged as a massless zero.
+template <int LPP, typename Smem>
+__device__ __forceinline__ void leaf_sum(const Smem& S, uint32_t k, uint32_t jself, bool me, bool soft, float2 px,
+                                         float2 py, float2 pz, float eps2, Sums& s, uint32_t sub) {
+  for (uint32_t j = 2 * sub; j < k; j += 2 * LPP) {
+    const bool u0 = me && (soft || j != jself), u1 = me && j + 1 < k && (soft || j + 1 != jself);
+    pair_step(S, 8 * j, px, py, pz, u0 ? eps2 : INFINITY, u1 ? eps2 : INFINITY, s);
+  }
+}
+
+// Direct sums of the queued leaves (nq of them, qp source pairs in all).
+//
+// What bounds it: an opened leaf is opened by a third of the item's 32 particles, so
+// a sum in which every lane takes every source of the leaf wastes two thirds of its
+// issue slots (a 32-particle item ran 453 packed steps for 162 useful ones per lane on
+// the 524288-particle disk, theta 0.5). Here the item's particles form subgroups of 8 Morton neighbours, and
+// the warp takes one subgroup at a time: 8 particles x 4 lanes, the lanes of a
+// particle splitting the source pairs that some particle of the subgroup takes part
+// in: 281 steps (subgroups of 16: 352, of 4: 229 with twice the subgroups to set up).
+// The price is one list of the subgroup's pairs and one sum over the 4 lanes per
+// subgroup and window, so leaves are queued until a window is nearly full (windows of
+// 64 pairs: walk 1027 us, of 96: 1000 us, of 32: 1103 us; 96 fills the shared memory
+// of 7 blocks per SM). Against the leaf-by-leaf sums it replaced: walk of that disk
+// 1091 -> 1000 us (49.7 -> 47.3 thousand warp instructions per item), the collision of
+// 524288 1140 -> 1087 us, 16384 particles (items of 8) 87 -> 75 us.
+//
+// A window: each lane turns its queued leaf into source pairs (a leaf of odd count
+// ends in a massless zero), then stages whole pairs, so the loads of a window are in
+// flight together and the staging stores are 128 bits wide.
+// Items of 8 or 4 particles are one subgroup: no list, and the lanes' partial sums stay
+// where the rest of the walk keeps them.
+template <int LPP, typename Smem>
+__device__ __forceinline__ void leaf_flush(Smem& S, const float4* __restrict__ pin, uint32_t nq, uint32_t qp,
+                                           uint32_t gbeg, int lane, bool soft, float eps2, float nx, float ny,
+                                           float nz, Sums& s) {
+  constexpr uint32_t G = 32 / LPP, SUBT = G < 8 ? G : 8, SH = 32 / SUBT, NSUB = G / SUBT;
+  constexpr uint32_t SMASK = (1u << SUBT) - 1u;
+  constexpr uint32_t W = kLeafWindow, kPer = W / 32;  // pairs a lane stages
+  const unsigned full = 0xffffffffu, below = (1u << lane) - 1u;
+  const uint32_t tl = lane % SUBT, share = lane / SUBT;
+  for (uint32_t w0 = 0; w0 < qp; w0 += W) {
+    __syncwarp();  // the queue is written; the staging is no longer read
+    uint32_t run = 0;
+    for (uint32_t e0 = 0; e0 < nq; e0 += 32) {
+      const bool has = e0 + lane < nq;
+      const uint2 en = has ? S.q[e0 + lane] : make_uint2(0u, 0u);
+      const uint32_t first = en.x & ((1u << kLeafCountShift) - 1u), cnt = (en.x >> kLeafCountShift) + 1u;
+      const uint32_t np = has ? (cnt + 1u) >> 1 : 0u;
+      uint32_t incl = np;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(full, incl, o);
+        if (lane >= o) incl += y;
+      }
+      // the leaf's pairs [klo, khi) lie in the window, pair k at window position at + k
+      const int at = (int)(run + incl - np - w0);
+      const int klo = max(0, -at), khi = min((int)np, (int)W - at);
+      const uint32_t kn = khi > klo ? (uint32_t)(khi - klo) : 0u;
+#pragma unroll
+      for (uint32_t k = 0; k < kLeafMax / 2; k++)
+        if (k - (uint32_t)klo < kn) S.pinfo[at + (int)k] = make_uint2((first + 2 * k) | 0x80000000u, en.y);
+      if ((cnt & 1u) && np - 1u - (uint32_t)klo < kn) S.pinfo[at + (int)np - 1].x = first + 2 * (np - 1u);
+      run += __shfl_sync(full, incl, 31);
+    }
+    __syncwarp();
+    const uint32_t nw = min(W, qp - w0);
+    uint32_t pm[kPer];
+    float4 A[kPer], B[kPer];
+    // all loads first (no branches): slots past the window repeat its last pair and
+    // no list names them; a missing second source is the first with no mass
+#pragma unroll
+    for (uint32_t r = 0; r < kPer; r++) {
+      const uint32_t t = lane + 32 * r;
+      const uint2 pi = S.pinfo[min(t, nw - 1)];
+      const float4* src = pin + 2 * (size_t)(pi.x & 0x7fffffffu);
+      const bool both = pi.x >> 31;
+      A[r] = __ldg(src);
+      B[r] = __ldg(src + (both ? 2 : 0));
+      B[r].w = both ? B[r].w : 0.f;
+      pm[r] = t < nw ? pi.y : 0u;
+    }
+#pragma unroll
+    for (uint32_t r = 0; r < kPer; r++) {
+      const uint32_t t = lane + 32 * r;
+      *reinterpret_cast<float4*>(&S.lxy[4 * t]) = make_float4(A[r].x, B[r].x, A[r].y, B[r].y);
+      *reinterpret_cast<float4*>(&S.lzm[4 * t]) = make_float4(A[r].z, B[r].z, A[r].w, B[r].w);
+    }
+#pragma unroll 1
+    for (uint32_t g = 0; g < NSUB; g++) {
+      uint32_t n = nw;
+      if (NSUB > 1) {  // the subgroup's pairs, in window order, padded with a pair nobody takes
+        n = 0;
+#pragma unroll
+        for (uint32_t r = 0; r < kPer; r++) {
+          const uint32_t m = (pm[r] >> (SUBT * g)) & SMASK;
+          const uint32_t b = __ballot_sync(full, m != 0u);
+          if (m) S.list[n + __popc(b & below)] = (16 * (lane + 32 * r)) | (m << 24);
+          n += __popc(b);
+        }
+        if (lane < (int)SH) S.list[n + lane] = 0u;
+      }
+      __syncwarp();
+      const float2 px = f2(NSUB > 1 ? __shfl_sync(full, nx, SUBT * g + tl) : nx);
+      const float2 py = f2(NSUB > 1 ? __shfl_sync(full, ny, SUBT * g + tl) : ny);
+      const float2 pz = f2(NSUB > 1 ? __shfl_sync(full, nz, SUBT * g + tl) : nz);
+      Sums z;
+      if (NSUB > 1) z.ax = z.ay = z.az = z.pt = f2(0.f);
+      else z = s;
+      if (soft) {
+        const uint32_t bit = NSUB > 1 ? 0x1000000u << tl : 1u << tl;
+#pragma unroll 2
+        for (uint32_t j0 = 0; j0 < n; j0 += SH) {
+          uint32_t at, m;
+          if (NSUB > 1) {
+            m = S.list[j0 + share];
+            at = m & 0xffffffu;
+          } else {
+            const uint32_t t = min(j0 + share, n - 1);
+            at = 16 * t;
+            m = j0 + share < n ? S.pinfo[t].y : 0u;
+          }
+          const float e = m & bit ? eps2 : INFINITY;
+          pair_step(S, at, px, py, pz, e, e, z);
+        }
+      } else {  // the particle's own source is left out
+        const uint32_t self = gbeg + SUBT * g + tl;
+        for (uint32_t j0 = 0; j0 < n; j0 += SH) {
+          uint32_t t = min(j0 + share, n - 1), m;
+          if (NSUB > 1) {
+            m = S.list[j0 + share];
+            t = (m & 0xffffffu) >> 4;
+            m >>= 24;
+          } else {
+            m = j0 + share < n ? S.pinfo[t].y : 0u;
+          }
+          const uint32_t fx = S.pinfo[t].x, f = fx & 0x7fffffffu;
+          const bool me = (m >> tl) & 1u;
+          pair_step(S, 16 * t, px, py, pz, me && f != self ? eps2 : INFINITY,
+                    me && (fx >> 31) && f + 1 != self ? eps2 : INFINITY, z);
+        }
+      }
+      if (NSUB > 1) {  // add the shares; the particle's own lane keeps the result
+        float v[4] = {z.ax.x + z.ax.y, z.ay.x + z.ay.y, z.az.x + z.az.y, z.pt.x + z.pt.y};
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+#pragma unroll
+          for (uint32_t o = SUBT; o < 32; o <<= 1) v[k] += __shfl_xor_sync(full, v[k], o);
+        }
+        if (lane / SUBT == g) {
+          s.ax.x += v[0];
+          s.ay.x += v[1];
+          s.az.x += v[2];
+          s.pt.x += v[3];
+        }
+        __syncwarp();  // the list is no longer read
+      } else {
+        s = z;
+      }
+    }
+  }
+}
 
 // Kahan step on packed pairs: s + x with the lost low-order part kept in c
 // (c holds the negated error; the compensated total is s - c).
@@ -323,11 +436,10 @@ __device__ __forceinline__ uint32_t warp_transpose(uint32_t x, int lane) {
 // terms (at most 32 per lane) are summed plainly and each round's sum is added to
 // the particle's total with a Kahan step; near-field leaf sums add plainly into
 // the same totals.
-// MINB: resident blocks per SM the register budget is compiled for.
 // LPP: lanes per particle (walk group of 32 / LPP particles); a launch walks the
 // galaxies whose SegDesc wlpp field equals LPP and skips the others' work items.
-template <bool SF, bool DBG, bool ONE, bool COMP, int MINB, int LPP>
-__global__ void __launch_bounds__(kWalkThreads, MINB) walk_kernel(WalkArgs a) {
+template <bool SF, bool DBG, bool ONE, bool COMP, int LPP>
+__global__ void __launch_bounds__(kWalkThreads, kWalkResident) walk_kernel(WalkArgs a) {
   static_assert(LPP == 1 || LPP == 2 || LPP == 4 || LPP == 8, "lanes per particle");
   constexpr uint32_t G = 32 / LPP;                         // particles per work item
   constexpr int NPP = 16 / LPP;                            // slot pairs a lane tests in a full round
@@ -379,9 +491,8 @@ __global__ void __launch_bounds__(kWalkThreads, MINB) walk_kernel(WalkArgs a) {
     const uint32_t i = gbeg + pl;
     const bool valid = i < seg_end;
     // Walk groups of 32 read the particle's record again for the integration at
-    // the end, so only its negated position stays live through the walk (the
-    // 64-register build then needs no spills; measured faster for pools, the
-    // same for one large galaxy); smaller groups keep it (measured faster there).
+    // the end, so only its negated position stays live through the walk; smaller
+    // groups keep it (measured faster there).
     constexpr bool kReload = LPP == 1;
     float4 p0 = make_float4(0.f, 0.f, 0.f, 0.f), p1 = p0;
     if (valid) {
@@ -389,10 +500,11 @@ __global__ void __launch_bounds__(kWalkThreads, MINB) walk_kernel(WalkArgs a) {
       if (!kReload) p1 = a.pin[2 * (size_t)i + 1];
     }
     const float2 px = f2(-p0.x), py = f2(-p0.y), pz = f2(-p0.z);  // negated: r = q + (-p)
-    float2 ax = f2(0.f), ay = f2(0.f), az = f2(0.f), pt = f2(0.f);
+    Sums F = {f2(0.f), f2(0.f), f2(0.f), f2(0.f)};
     float2 cax = f2(0.f), cay = f2(0.f), caz = f2(0.f), cpt = f2(0.f);  // COMP only
     float dens = 0.f, selfw = 0.f;
     unsigned long long nmono = 0, npair = 0, nvisit = 0;
+    uint32_t nq = 0, qp = 0;  // queued leaves, their source pairs
     const unsigned all = __ballot_sync(full, valid) & GMASK;  // the item's particles (lanes of share 0)
 
     // Split walk: the first level of at least kSplitMinNodes nodes per split is
@@ -421,7 +533,12 @@ __global__ void __launch_bounds__(kWalkThreads, MINB) walk_kernel(WalkArgs a) {
     if (lane == 0) S.stack[0] = make_uint2(sd.node_off, all);  // the root: range {node_off, 1}
     sp = idle ? 0 : 1;
     uint32_t budget = 4u * sd.node_cap + 1024u;
-    while (sp > 0) {
+    while (true) {
+      if (qp >= (uint32_t)kLeafFlush || (sp == 0 && qp > 0)) {
+        leaf_flush<LPP>(S, a.pin, nq, qp, gbeg, lane, soft, eps2, px.x, py.x, pz.x, F);
+        nq = qp = 0;
+      }
+      if (sp == 0) break;
       __syncwarp();
       // pop up to kWalkRanges ranges; their children are staged and tested together
       const int nr = min(sp, kWalkRanges);
@@ -439,6 +556,8 @@ __global__ void __launch_bounds__(kWalkThreads, MINB) walk_kernel(WalkArgs a) {
       // (size^2 < eps^2/4, always accepted, nbody_bh.wgsl:112) get size^2 = -inf,
       // so the per-lane test is the single compare size^2 < theta^2 (r^2 + eps^2).
       bool own = false, isleaf = false, massive = false, skip = false;
+      uint32_t cnode = 0, cchild = 0, ccnt = 0;  // this lane's slot: node, first child or particle, count
+      float csize = 1.f;
       if (lane < 8 * kWalkRanges) {
         const int r = lane >> 3;
         const uint32_t c = lane & 7;
@@ -460,11 +579,14 @@ __global__ void __launch_bounds__(kWalkThreads, MINB) walk_kernel(WalkArgs a) {
           q = __ldg(&a.cm[rs + c]);
           w = a.info[rs + c];
         }
-        const uint32_t wc = w.info & ~kLeafBit;
+        cnode = rs + c;
+        cchild = w.child;
+        ccnt = w.info & ~kLeafBit;
+        csize = w.size;
         isleaf = real && (w.info & kLeafBit);
         massive = real && q.w != 0.0f && counted;
         skip = isleaf && !counted;
-        own = isleaf && q.w != 0.0f && w.child < gend && w.child + wc > gbeg;
+        own = isleaf && q.w != 0.0f && cchild < gend && cchild + ccnt > gbeg;
         float s2 = w.s2;
         if (q.w == 0.0f) {  // never opened, contributes nothing (far away, massless)
           s2 = -INFINITY;
@@ -478,10 +600,6 @@ __global__ void __launch_bounds__(kWalkThreads, MINB) walk_kernel(WalkArgs a) {
         S.czm[st] = q.z;
         S.czm[st + 2] = counted ? q.w : 0.0f;  // tested for opening, adds nothing
         S.cs2[lane] = s2;
-        S.cnode[lane] = rs + c;
-        S.cmeta[lane] = make_uint4(w.child, w.info,
-                                   own ? __float_as_uint(w.size) : 0u,
-                                   massive ? 1u : 0u);
       }
       const unsigned ownmask = __ballot_sync(full, own);  // leaves holding our particles
       const unsigned leafmask = __ballot_sync(full, isleaf);
@@ -539,17 +657,17 @@ __global__ void __launch_bounds__(kWalkThreads, MINB) walk_kernel(WalkArgs a) {
           raz = __ffma2_rn(rz, f, raz);
           rpt = __fadd2_rn(rpt, mr);
         } else {
-          ax = __ffma2_rn(rx, f, ax);
-          ay = __ffma2_rn(ry, f, ay);
-          az = __ffma2_rn(rz, f, az);
-          pt = __fadd2_rn(pt, mr);  // sum of m/r; potential = -G * sum
+          F.ax = __ffma2_rn(rx, f, F.ax);
+          F.ay = __ffma2_rn(ry, f, F.ay);
+          F.az = __ffma2_rn(rz, f, F.az);
+          F.pt = __fadd2_rn(F.pt, mr);  // sum of m/r; potential = -G * sum
         }
       }
       if (COMP) {
-        kahan_add2(ax, cax, rax);
-        kahan_add2(ay, cay, ray);
-        kahan_add2(az, caz, raz);
-        kahan_add2(pt, cpt, rpt);
+        kahan_add2(F.ax, cax, rax);
+        kahan_add2(F.ay, cay, ray);
+        kahan_add2(F.az, caz, raz);
+        kahan_add2(F.pt, cpt, rpt);
       }
       obits &= keep;
       const uint32_t om = __reduce_or_sync(full, obits);  // children opened by some lane
@@ -559,11 +677,12 @@ __global__ void __launch_bounds__(kWalkThreads, MINB) walk_kernel(WalkArgs a) {
       }
       for (uint32_t bb = ownmask; bb; bb &= bb - 1) {  // own-leaf density (nbody_bh.wgsl:93-95)
         const uint32_t cc = __ffs(bb) - 1;
-        const uint4 mt = S.cmeta[cc];
-        const uint32_t cnt = mt.y & ~kLeafBit;
-        if (((actbits >> (cc >> 3)) & 1u) && (i - mt.x) < cnt) {
-          const float sz = __uint_as_float(mt.z);
+        const uint32_t lf = __shfl_sync(full, cchild, cc), cnt = __shfl_sync(full, ccnt, cc);
+        const float sz = __shfl_sync(full, csize, cc);
+        if (((actbits >> (cc >> 3)) & 1u) && (i - lf) < cnt) {
           dens = (float)cnt / (sz * sz * sz);
+          // the leaf's direct sum includes the particle itself (softened walks)
+          if (((obits & ~skipm) >> cc) & 1u) selfw += 1.0f;
         }
       }
       if (!om) continue;
@@ -580,11 +699,9 @@ __global__ void __launch_bounds__(kWalkThreads, MINB) walk_kernel(WalkArgs a) {
         bool ok = false;
         uint2 ent = make_uint2(0u, 0u);
         if ((pushc >> lane) & 1u) {
-          const uint4 mt = S.cmeta[lane];
-          const uint32_t cchild = mt.x, ccnt = mt.y & ~kLeafBit;
           // a galaxy's child ranges stay in its node range by construction (build,
           // upload check); the walk itself only guards the pool bounds
-          ok = cchild > S.cnode[lane] && (uint64_t)cchild + ccnt <= a.node_pool && ccnt >= 1u && ccnt <= 8u;
+          ok = cchild > cnode && ccnt - 1u < 8u && cchild <= a.node_pool - ccnt;
           if (!ok) raise_err(sst, GS_DERR_TREE);
           ent = make_uint2(cchild | ((ccnt - 1u) << 29), col);
         }
@@ -595,182 +712,69 @@ __global__ void __launch_bounds__(kWalkThreads, MINB) walk_kernel(WalkArgs a) {
         if (sp + np > kWalkStack && lane == 0) raise_err(sst, GS_DERR_STACK);  // not for depth <= 10 trees
         sp = min(sp + np, kWalkStack);
       }
-      // Opened leaves: direct sums, two sources at a time.
+      // Opened leaves: those of at most kLeafMax particles join the queue, in slot
+      // order; larger ones (coincident particles at the deepest level) are summed
+      // at once, in chunks of 32.
       const uint32_t leafc = om & leafmask & ~skipm;
-      // Walk groups of 32: leaves of <= 16 particles get their batch entries from
-      // their slots' lanes and are staged four per batch (one load round), each in
-      // a block of 16 sources; larger ones go in chunks of 32.
-      uint32_t big = 0;
-      if (LPP == 1 && leafc) {
+      if (leafc) {
         bool sm = false, bg = false;
-        uint4 ent = make_uint4(0u, 0u, 0u, 0u);
+        uint2 ent = make_uint2(0u, 0u);
+        uint32_t np = 0;
         if ((leafc >> lane) & 1u) {
-          const uint4 mt = S.cmeta[lane];
-          const uint32_t ccnt = mt.y & ~kLeafBit;
-          if ((uint64_t)mt.x + ccnt > a.pool_n) {
+          if (ccnt > a.pool_n || cchild > a.pool_n - ccnt) {
             raise_err(sst, GS_DERR_TREE);
           } else {
-            bg = ccnt > 16u;
-            sm = !bg;
-            ent = make_uint4(mt.x, ccnt, col, 0u);
+            bg = ccnt > kLeafMax;
+            sm = !bg && ccnt > 0u;  // an empty leaf adds nothing
+            ent = make_uint2(cchild | ((ccnt - 1u) << kLeafCountShift), col);
+            if (sm) np = (ccnt + 1u) >> 1;
           }
         }
         const uint32_t smallm = __ballot_sync(full, sm);
-        big = __ballot_sync(full, bg);
-        __syncwarp();  // earlier leaf sums are done reading the batch entries
-        if (sm) S.bl[__popc(smallm & ((1u << lane) - 1u))] = ent;
-        const uint32_t nsmall = __popc(smallm);
-        for (uint32_t b0 = 0; b0 < nsmall; b0 += 4) {
-          const uint32_t nb = min(4u, nsmall - b0);
-          __syncwarp();
-#pragma unroll
-          for (int r = 0; r < 2; r++) {
-            const uint32_t e = lane + 32 * r, slot = e >> 4, q = e & 15u;
-            if (slot < nb) {
-              const uint4 bl = S.bl[b0 + slot];
-              float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-              if (q < bl.y) v = __ldg(&a.pin[2 * (size_t)(bl.x + q)]);
-              const uint32_t se = 4 * (e >> 1) + (e & 1);
-              S.lxy[se] = v.x;
-              S.lxy[se + 2] = v.y;
-              S.lzm[se] = v.z;
-              S.lzm[se + 2] = v.w;
-            }
-          }
-          __syncwarp();
-          for (uint32_t sl = 0; sl < nb; sl++) {
-            const uint4 bl = S.bl[b0 + sl];
-            leaf_sum<LPP>(S, 16 * sl, bl.y, bl.y, i - bl.x, (bl.z >> pl) & 1u, soft, px, py, pz, eps2, ax, ay,
-                          az, pt, selfw, npair, DBG, sub);
+        if (sm) S.q[nq + __popc(smallm & ((1u << lane) - 1u))] = ent;
+        nq += __popc(smallm);
+        qp += __reduce_add_sync(full, np);
+        if (DBG) {
+          for (uint32_t bb = leafc; bb; bb &= bb - 1) {
+            const uint32_t cc = __ffs(bb) - 1;
+            const unsigned open = __shfl_sync(full, col, cc);
+            const uint32_t lf = __shfl_sync(full, cchild, cc), cnt = __shfl_sync(full, ccnt, cc);
+            if (sub == 0 && ((open >> pl) & 1u)) npair += cnt - (i - lf < cnt ? 1u : 0u);
           }
         }
-      }
-      for (uint32_t bb = big; bb; bb &= bb - 1) {
-        const uint32_t cc = __ffs(bb) - 1;
-        const unsigned open = __shfl_sync(full, col, cc);
-        const uint4 mt = S.cmeta[cc];
-        const uint32_t cchild = mt.x, ccnt = mt.y & ~kLeafBit;
-        for (uint32_t b0 = 0; b0 < ccnt; b0 += 32) {
-          const uint32_t k = min(32u, ccnt - b0);
-          __syncwarp();
-          float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (lane < (int)k) v = __ldg(&a.pin[2 * (size_t)(cchild + b0 + lane)]);
-          const int se = 4 * (lane >> 1) + (lane & 1);
-          S.lxy[se] = v.x;
-          S.lxy[se + 2] = v.y;
-          S.lzm[se] = v.z;
-          S.lzm[se + 2] = v.w;
-          if (lane == 0) S.lxy[64] = S.lxy[66] = S.lzm[64] = S.lzm[66] = 0.f;  // source 32
-          __syncwarp();
-          leaf_sum<LPP>(S, 0, k, k, i - (cchild + b0), (open >> pl) & 1u, soft, px, py, pz, eps2, ax, ay,
-                        az, pt, selfw, npair, DBG, sub);
-        }
-      }
-      // Walk groups of 16 or fewer (a particle's pairs split over LPP lanes): the
-      // round's opened leaves lie back to back in slot order in a space of source
-      // pairs (leaf k at pairs [P_k, P_k + ceil(n_k / 2))), staged and summed in
-      // batches of 32 pairs, so every lane's share of a batch is whole pairs of
-      // leaf sources and no step is spent on a leaf's unused staging slots.
-      if (LPP > 1 && leafc) {
-        bool lf = false;
-        uint32_t lfirst = 0, lcnt = 0, lnp = 0;
-        if ((leafc >> lane) & 1u) {
-          const uint4 mt = S.cmeta[lane];
-          lfirst = mt.x;
-          lcnt = mt.y & ~kLeafBit;
-          if ((uint64_t)lfirst + lcnt > a.pool_n) {
-            raise_err(sst, GS_DERR_TREE);
-          } else {
-            lf = lcnt > 0u;  // an empty leaf adds nothing
-            lnp = (lcnt + 1u) >> 1;
-          }
-        }
-        uint32_t incl = lnp;  // inclusive prefix of the pair counts over the slots
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const uint32_t y = __shfl_up_sync(full, incl, o);
-          if (lane >= o) incl += y;
-        }
-        const uint32_t P = incl - lnp, T = __shfl_sync(full, incl, 31);
-        const uint32_t lfm = __ballot_sync(full, lf);
-        // item particles that opened the leaf holding them (the self pair)
-        uint32_t selfm = 0;
-        if (lf) {
-          const uint32_t lo = max(lfirst, gbeg), hi = min(lfirst + lcnt, gend);
-          if (lo < hi) {
-            const uint32_t b0 = lo - gbeg, b1 = hi - gbeg;  // item particle positions [b0, b1)
-            selfm = col & ((b1 >= 32u ? 0xffffffffu : (1u << b1) - 1u) & ~((1u << b0) - 1u));
-          }
-        }
-        const bool selfhit = (__reduce_or_sync(full, selfm) >> pl) & 1u;
-        if (soft && sub == 0 && selfhit) selfw += 1.0f;
-        __syncwarp();  // the previous round's batches are done reading the table and staging
-        if (lf) S.bl[__popc(lfm & ((1u << lane) - 1u))] = make_uint4(lfirst, lcnt, col, P);
-        __syncwarp();
-        uint32_t selfsrc = 0xffffffffu;  // without softening: the self source in pair space
-        if (DBG || !soft) {
-          const uint32_t nl = __popc(lfm);
-          for (uint32_t k = 0; k < nl; k++) {
-            const uint4 L = S.bl[k];
-            if ((L.z >> pl) & 1u) {
-              const bool in = i - L.x < L.y;
-              if (in) selfsrc = 2 * L.w + (i - L.x);
-              if (DBG && sub == 0) npair += L.y - (in ? 1u : 0u);
-            }
-          }
-        }
-        for (uint32_t w0 = 0; w0 < T; w0 += 32) {
-          // leaves starting in this batch's window of pairs, and those before it
-          const uint32_t Wb = __reduce_or_sync(full, lf && P >= w0 && P - w0 < 32u ? 1u << (P - w0) : 0u);
-          const uint32_t base = __popc(__ballot_sync(full, lf && P < w0));
-          if (w0) __syncwarp();  // the previous batch's sums are done reading the staging
-          // stage source e = lane + 32 r of the batch: pair t = e / 2 of leaf k
-#pragma unroll
-          for (int r = 0; r < 2; r++) {
-            const uint32_t e = lane + 32 * r, t = e >> 1;
+        for (uint32_t bb = __ballot_sync(full, bg); bb; bb &= bb - 1) {
+          const uint32_t cc = __ffs(bb) - 1;
+          const unsigned open = __shfl_sync(full, col, cc);
+          const uint32_t lf = __shfl_sync(full, cchild, cc), cnt = __shfl_sync(full, ccnt, cc);
+          for (uint32_t b0 = 0; b0 < cnt; b0 += 32) {
+            const uint32_t k = min(32u, cnt - b0);
+            __syncwarp();
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (w0 + t < T) {
-              const uint4 L = S.bl[base + __popc(Wb & (0xffffffffu >> (31 - t))) - 1];
-              const uint32_t q = 2 * (w0 + t - L.w) + (e & 1u);  // source within the leaf
-              if (q < L.y) v = __ldg(&a.pin[2 * (size_t)(L.x + q)]);
-            }
-            const uint32_t se = 4 * t + (e & 1u);
+            if (lane < (int)k) v = __ldg(&a.pin[2 * (size_t)(lf + b0 + lane)]);
+            const int se = 4 * (lane >> 1) + (lane & 1);
             S.lxy[se] = v.x;
             S.lxy[se + 2] = v.y;
             S.lzm[se] = v.z;
             S.lzm[se + 2] = v.w;
+            __syncwarp();
+            leaf_sum<LPP>(S, k, i - (lf + b0), (open >> pl) & 1u, soft, px, py, pz, eps2, F, sub);
           }
-          // lane t answers for pair t: the item particles that opened its leaf
-          // (copied to every share when LPP > 1); transposed, each lane holds the
-          // pairs its particle takes part in
-          uint32_t mt = 0;
-          if (w0 + lane < T) mt = S.bl[base + __popc(Wb & (0xffffffffu >> (31 - lane))) - 1].z;
-          if (LPP == 2) mt *= 0x00010001u;
-          if (LPP == 4) mt *= 0x01010101u;
-          if (LPP == 8) mt *= 0x11111111u;
-          const uint32_t pm = warp_transpose(mt, lane) >> sub;
-          const uint32_t nbp = min(32u, T - w0);
-          __syncwarp();
-          if (soft)
-            leaf_batch<LPP, true>(S, nbp, pm, 0u, px, py, pz, eps2, ax, ay, az, pt, sub);
-          else
-            leaf_batch<LPP, false>(S, nbp, pm, selfsrc - 2 * w0, px, py, pz, eps2, ax, ay, az, pt, sub);
         }
       }
     }
     if (COMP) {  // fold the compensations into the sums
-      ax = __ffma2_rn(cax, f2(-1.0f), ax);
-      ay = __ffma2_rn(cay, f2(-1.0f), ay);
-      az = __ffma2_rn(caz, f2(-1.0f), az);
-      pt = __ffma2_rn(cpt, f2(-1.0f), pt);
+      F.ax = __ffma2_rn(cax, f2(-1.0f), F.ax);
+      F.ay = __ffma2_rn(cay, f2(-1.0f), F.ay);
+      F.az = __ffma2_rn(caz, f2(-1.0f), F.az);
+      F.pt = __ffma2_rn(cpt, f2(-1.0f), F.pt);
     }
     if (LPP > 1) {  // add the shares of each particle (lanes pl, pl + G, ...), fixed order
 #pragma unroll
       for (uint32_t o = G; o < 32; o <<= 1) {
-        ax = __fadd2_rn(ax, make_float2(__shfl_xor_sync(full, ax.x, o), __shfl_xor_sync(full, ax.y, o)));
-        ay = __fadd2_rn(ay, make_float2(__shfl_xor_sync(full, ay.x, o), __shfl_xor_sync(full, ay.y, o)));
-        az = __fadd2_rn(az, make_float2(__shfl_xor_sync(full, az.x, o), __shfl_xor_sync(full, az.y, o)));
-        pt = __fadd2_rn(pt, make_float2(__shfl_xor_sync(full, pt.x, o), __shfl_xor_sync(full, pt.y, o)));
+        F.ax = __fadd2_rn(F.ax, make_float2(__shfl_xor_sync(full, F.ax.x, o), __shfl_xor_sync(full, F.ax.y, o)));
+        F.ay = __fadd2_rn(F.ay, make_float2(__shfl_xor_sync(full, F.ay.x, o), __shfl_xor_sync(full, F.ay.y, o)));
+        F.az = __fadd2_rn(F.az, make_float2(__shfl_xor_sync(full, F.az.x, o), __shfl_xor_sync(full, F.az.y, o)));
+        F.pt = __fadd2_rn(F.pt, make_float2(__shfl_xor_sync(full, F.pt.x, o), __shfl_xor_sync(full, F.pt.y, o)));
         selfw += __shfl_xor_sync(full, selfw, o);
       }
     }
@@ -794,7 +798,7 @@ __global__ void __launch_bounds__(kWalkThreads, MINB) walk_kernel(WalkArgs a) {
       const uint32_t li = i - sd.off;
       const size_t st = a.split_stride;
       float4* const B = a.split_buf;
-      const float4 o0 = make_float4(ax.x, ax.y, ay.x, ay.y), o1 = make_float4(az.x, az.y, pt.x, pt.y);
+      const float4 o0 = make_float4(F.ax.x, F.ax.y, F.ay.x, F.ay.y), o1 = make_float4(F.az.x, F.az.y, F.pt.x, F.pt.y);
       const float4 o2 = make_float4(dens, selfw, 0.f, 0.f);
       if (valid && sub == 0) {
         B[(size_t)ksp * st + li] = o0;
@@ -829,10 +833,10 @@ __global__ void __launch_bounds__(kWalkThreads, MINB) walk_kernel(WalkArgs a) {
             u2 = make_float4(fmaxf(u2.x, v2.x), u2.y + v2.y, 0.f, 0.f);  // the own leaf is found once or equal
           }
         }
-        ax = make_float2(u0.x, u0.y);
-        ay = make_float2(u0.z, u0.w);
-        az = make_float2(u1.x, u1.y);
-        pt = make_float2(u1.z, u1.w);
+        F.ax = make_float2(u0.x, u0.y);
+        F.ay = make_float2(u0.z, u0.w);
+        F.az = make_float2(u1.x, u1.y);
+        F.pt = make_float2(u1.z, u1.w);
         dens = u2.x;
         selfw = u2.y;
       }
@@ -841,13 +845,13 @@ __global__ void __launch_bounds__(kWalkThreads, MINB) walk_kernel(WalkArgs a) {
       p0 = a.pin[2 * (size_t)i];
       p1 = a.pin[2 * (size_t)i + 1];
     }
-    if (soft && selfw != 0.0f) pt.x -= selfw * p0.w * rsqrtf(eps2);
+    if (soft && selfw != 0.0f) F.pt.x -= selfw * p0.w * rsqrtf(eps2);
 
     double e_diag = 0, e_true = 0, mx = 0, my = 0, mz = 0, ms = 0;
     if (valid && sub == 0) {
       const float G = P.G;
-      float fx = (ax.x + ax.y) * G, fy = (ay.x + ay.y) * G, fz = (az.x + az.y) * G;
-      const float pot = -(pt.x + pt.y) * G;
+      float fx = (F.ax.x + F.ax.y) * G, fy = (F.ay.x + F.ay.y) * G, fz = (F.az.x + F.az.y) * G;
+      const float pot = -(F.pt.x + F.pt.y) * G;
       if (DBG) {
         a.dbg_acc[i] = make_float4(fx, fy, fz, pot);
         a.dbg_dens[i] = dens;
