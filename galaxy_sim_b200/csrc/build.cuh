@@ -297,6 +297,47 @@ enum ComMode : int {
   kComF64 = 2,   // FP32 leaves, FP64 internal nodes (large-node reduction in double)
 };
 
+// Mass and centre of mass in the order of the additions: FP32 (refresh_level's
+// arithmetic) or FP64 rounded at the end.
+template <bool F64>
+struct ComSum {
+  float mm = 0, cx = 0, cy = 0, cz = 0;
+  __device__ __forceinline__ void add(float4 q) {
+    cx = fmaf(q.x, q.w, cx);
+    cy = fmaf(q.y, q.w, cy);
+    cz = fmaf(q.z, q.w, cz);
+    mm += q.w;
+  }
+  __device__ __forceinline__ float4 mean() const {
+    return mm > 0.0f ? make_float4(cx / mm, cy / mm, cz / mm, mm) : make_float4(0.f, 0.f, 0.f, mm);
+  }
+};
+template <>
+struct ComSum<true> {
+  double mm = 0, cx = 0, cy = 0, cz = 0;
+  __device__ __forceinline__ void add(float4 q) {
+    const double qm = q.w;
+    mm = __dadd_rn(mm, qm);
+    cx = __dadd_rn(cx, __dmul_rn((double)q.x, qm));
+    cy = __dadd_rn(cy, __dmul_rn((double)q.y, qm));
+    cz = __dadd_rn(cz, __dmul_rn((double)q.z, qm));
+  }
+  __device__ __forceinline__ float4 mean() const {
+    return mm > 0 ? make_float4(__double2float_rn(cx / mm), __double2float_rn(cy / mm),
+                                __double2float_rn(cz / mm), __double2float_rn(mm))
+                  : make_float4(0.f, 0.f, 0.f, __double2float_rn(mm));
+  }
+};
+
+__device__ __forceinline__ WalkInfo walk_info(float size, uint32_t child, uint32_t info) {
+  WalkInfo w;
+  w.s2 = size * size;
+  w.child = child;
+  w.info = info;
+  w.size = size;
+  return w;
+}
+
 // K4: one thread per leaf slot (a block per build tile, kLeafThreads = one
 // tile); leaf COM, then carry each finished node to its parent; the last child
 // to finish sums the parent (children in slot order).
@@ -360,7 +401,7 @@ __global__ void __launch_bounds__(kLeafThreads)
       c = make_float4(__double2float_rn(__dmul_rn(cx, inv)), __double2float_rn(__dmul_rn(cy, inv)),
                       __double2float_rn(__dmul_rn(cz, inv)), __double2float_rn(mm));
     } else {
-      float mm = 0, cx = 0, cy = 0, cz = 0;
+      ComSum<false> sum;
       for (uint32_t j0 = lo; j0 < hi; j0 += kComChunk) {
         float4 q[kComChunk];
 #pragma unroll
@@ -369,21 +410,13 @@ __global__ void __launch_bounds__(kLeafThreads)
 #pragma unroll
         for (int k = 0; k < kComChunk; k++) {
           if (j0 + k >= hi) break;
-          cx = fmaf(q[k].x, q[k].w, cx);
-          cy = fmaf(q[k].y, q[k].w, cy);
-          cz = fmaf(q[k].z, q[k].w, cz);
-          mm += q[k].w;
+          sum.add(q[k]);
         }
       }
-      c = mm > 0.0f ? make_float4(cx / mm, cy / mm, cz / mm, mm) : make_float4(0.f, 0.f, 0.f, mm);
+      c = sum.mean();
     }
     b.cm[n] = c;
-    WalkInfo w;
-    w.s2 = size * size;
-    w.child = lo;
-    w.info = kLeafBit | (hi - lo);
-    w.size = size;
-    b.info[n] = w;
+    b.info[n] = walk_info(size, lo, kLeafBit | (hi - lo));
     // carry upwards
     while (p >= 0) {
       const uint32_t up = (uint32_t)p;
@@ -420,18 +453,7 @@ __global__ void __launch_bounds__(kLeafThreads)
 #pragma unroll
       for (int k = 0; k < 8; k++) q[k] = k < (int)nc ? __ldcg(&b.cm[cb + k]) : make_float4(0.f, 0.f, 0.f, 0.f);
       float4 pc;
-      if (MODE == kComF32) {
-        float mm = 0, cx = 0, cy = 0, cz = 0;
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-          if (k >= (int)nc) break;
-          cx = fmaf(q[k].x, q[k].w, cx);
-          cy = fmaf(q[k].y, q[k].w, cy);
-          cz = fmaf(q[k].z, q[k].w, cz);
-          mm += q[k].w;
-        }
-        pc = mm > 0.0f ? make_float4(cx / mm, cy / mm, cz / mm, mm) : make_float4(0.f, 0.f, 0.f, mm);
-      } else {
+      if (MODE == kComJs) {
         double mm = 0, cx = 0, cy = 0, cz = 0;
 #pragma unroll
         for (int k = 0; k < 8; k++) {
@@ -442,25 +464,21 @@ __global__ void __launch_bounds__(kLeafThreads)
           cy = __dadd_rn(cy, __dmul_rn((double)q[k].y, qm));
           cz = __dadd_rn(cz, __dmul_rn((double)q[k].z, qm));
         }
-        if (MODE == kComJs) {
-          const double inv = mm > 0 ? __ddiv_rn(1.0, mm) : 0.0;
-          pc = make_float4(__double2float_rn(__dmul_rn(cx, inv)),
-                           __double2float_rn(__dmul_rn(cy, inv)),
-                           __double2float_rn(__dmul_rn(cz, inv)), __double2float_rn(mm));
-        } else {
-          pc = mm > 0 ? make_float4(__double2float_rn(cx / mm), __double2float_rn(cy / mm),
-                                    __double2float_rn(cz / mm), __double2float_rn(mm))
-                      : make_float4(0.f, 0.f, 0.f, __double2float_rn(mm));
+        const double inv = mm > 0 ? __ddiv_rn(1.0, mm) : 0.0;
+        pc = make_float4(__double2float_rn(__dmul_rn(cx, inv)), __double2float_rn(__dmul_rn(cy, inv)),
+                         __double2float_rn(__dmul_rn(cz, inv)), __double2float_rn(mm));
+      } else {
+        ComSum<MODE == kComF64> sum;
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+          if (k >= (int)nc) break;
+          sum.add(q[k]);
         }
+        pc = sum.mean();
       }
       const float psize = __double2float_rn(ldexp(m.root_size, -dp));
       b.cm[up] = pc;
-      WalkInfo pw;
-      pw.s2 = psize * psize;
-      pw.child = cb;
-      pw.info = nc;
-      pw.size = psize;
-      b.info[up] = pw;
+      b.info[up] = walk_info(psize, cb, nc);
       n = up;
       p = pp;
     }

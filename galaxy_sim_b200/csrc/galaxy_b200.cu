@@ -29,6 +29,7 @@
 
 #include "build.cuh"
 #include "common.cuh"
+#include "fused.cuh"
 #include "morton.cuh"
 #include "particles.cuh"
 #include "sort.cuh"
@@ -245,6 +246,7 @@ struct gs_ctx {
   int walk_group = 32;             // tuning: walk group size (0: by galaxy size; 4, 8, 16 or 32 particles)
   int walk_split = 1;              // tuning: walk splits per work item of a lone galaxy (0: by its size; 1, 2, 4, 8)
   uint32_t walk_items[4] = {0, 0, 0, 0};  // work items per lanes-per-particle class (1, 2, 4, 8)
+  bool fuse_ok = false;    // the layout's galaxy is rebuilt by one kernel on one cluster
   bool walk_comp = false;  // compensated far-field sums in the walk (a Kahan step per round)
   // pinned staging of Params uploads: a ring of entries, each rewritten only after
   // the copy that last read it has run (its event), so an update does not wait
@@ -345,6 +347,53 @@ struct gs_ctx {
   if (!s) return (ctx)->fail(GS_ENOTREADY, "no galaxy in selected slot %u", (ctx)->sel);
 
 namespace {
+
+using FuseKernel = void (*)(FuseArgs);
+FuseKernel fuse_kernel(int com_mode, uint32_t threads) {
+  if (com_mode == kComF64)
+    return threads == 256 ? fused_rebuild_kernel<kComF64, 256> : fused_rebuild_kernel<kComF64, 512>;
+  return threads == 256 ? fused_rebuild_kernel<kComF32, 256> : fused_rebuild_kernel<kComF32, 512>;
+}
+
+void fuse_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute attr[2], const FuseShape& f, cudaStream_t s) {
+  cfg = {};
+  cfg.gridDim = dim3(f.ctas);
+  cfg.blockDim = dim3(f.threads);
+  cfg.dynamicSmemBytes = fuse_smem(f.log2p);
+  cfg.stream = s;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = f.ctas;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+}
+
+// Whether the current device runs the one-cluster rebuild of n particles (a cluster of
+// that many blocks with their shared memory fits); opts its kernels into the size.
+bool fuse_supported(uint32_t n) {
+  if (n > kFuseMax) return false;
+  const FuseShape f = fuse_shape(n);
+  for (int mode : {(int)kComF32, (int)kComF64}) {
+    const void* k = (const void*)fuse_kernel(mode, f.threads);
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[2];
+    fuse_config(cfg, attr, f, nullptr);
+    cfg.numAttrs = 1;  // the cluster shape
+    int clusters = 0;
+    // the largest block of this thread count, so that a smaller galaxy's call does not lower it
+    const uint32_t lp = f.threads == 256 ? 10u : 11u;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fuse_smem(lp));
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&clusters, k, &cfg);
+    if (e != cudaSuccess || clusters < 1) {
+      cudaGetLastError();  // the rebuild then runs as separate kernels
+      return false;
+    }
+  }
+  return true;
+}
 
 int pool_init(gs_ctx* c, int device, uint64_t cap, uint32_t slots) {
   c->device = device;
@@ -566,6 +615,7 @@ int ensure_layout(gs_ctx* c) {
   c->walk_grid = std::min<uint32_t>(std::max<uint32_t>(1, cdiv(most, kWalkWarps)),
                                     (uint32_t)c->sms * std::min(c->walk_bps, kWalkResident));
   for (int k = 0; k < 4; k++) c->walk_items[k] = items[k];
+  c->fuse_ok = h.size() == 1 && fuse_supported(h[0].n);
   c->drop_graphs();
   c->lay_dirty = false;
   return GS_OK;
@@ -702,10 +752,39 @@ void enqueue_walk(gs_ctx* c, int sf) {
   c->cur ^= 1;
 }
 
+// The rebuild of one small galaxy as one kernel on one cluster.
+void enqueue_fused_rebuild(gs_ctx* c, int advance_time, bool track) {
+  FuseArgs a;
+  a.pin = c->part[c->cur];
+  a.pout = c->part[c->cur ^ 1];
+  a.sin = c->stel[c->scur];
+  a.sout = c->stel[c->scur ^ 1];
+  a.keys = c->keys[0];
+  a.vals = c->vals[0];
+  a.frames = c->frames;
+  a.st = c->st;
+  a.b = c->bb();
+  a.sd = c->seg_host[0];
+  const FuseShape f = fuse_shape(a.sd.n);
+  a.log2p = f.log2p;
+  a.advance_time = advance_time;
+  a.track = track ? 1 : 0;
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attr[2];
+  fuse_config(cfg, attr, f, c->stream);
+  cudaLaunchKernelEx(&cfg, fuse_kernel(c->com_mode, f.threads), a);
+}
+
 // codes + sort + gather (+ tracking/EMA) + build + refresh; flips cur and scur.
 void enqueue_sort_build(gs_ctx* c, int advance_time) {
   const bool track = c->any_tracking();
   const Layout& L = c->lay;
+  if (c->fuse_ok) {
+    enqueue_fused_rebuild(c, advance_time, track);
+    c->cur ^= 1;
+    c->scur ^= 1;
+    return;
+  }
   enqueue_codes_sort(c, c->part[c->cur], 2, advance_time);
   enqueue_sort_passes(c, track);
   launch_pdl(gather_kernel, L.flag_tiles, kTileThreads, c->stream, (const uint32_t*)c->vals[0],

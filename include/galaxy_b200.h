@@ -127,7 +127,8 @@ int gs_set_walk_mode(gs_ctx* ctx, int compensated);
  * changes results.
  * GS_TUNE_SORT_ITEMS = keys per thread of a sort tile (4, 8 or 16, or 0 = by the
  * largest galaxy's size: 4 up to 131072 particles, 8 up to 393216, else 16;
- * default 0 for a gs_create context, 16 for a pool); never
+ * default 0 for a gs_create context, 16 for a pool; a lone galaxy of at most 32768
+ * particles is rebuilt by one kernel that has no tiles); never
  * changes results (a stable sort has one answer).
  * GS_TUNE_WALK_GROUP = particles a warp walks together: 32 (one lane per particle),
  * 16, 8 or 4 (two, four or eight lanes per particle, splitting its node tests and
