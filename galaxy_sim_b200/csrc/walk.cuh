@@ -63,7 +63,7 @@ constexpr int kWalkStack = 8 * 11 * kWalkRanges;
 // sums were queued, a second build of 64 registers for 8 blocks ran the 96-galaxy
 // pool in 7.569 ms against 7.572 ms for this one.)
 constexpr int kWalkBlocksPerSM = 8;
-constexpr int kWalkResident = 7;
+constexpr int kWalkResident = 7;  // 6 with compensated sums (80 registers: 306 -> 290 us on a sphere of 200003)
 constexpr uint32_t kWalkGroup = 32;             // particles per walk group (layout, diagnostics)
 constexpr uint32_t kWalkParts = 8;              // partial-sum slots per walk group (the largest LPP)
 // with the walk group chosen by size, galaxies of at most this many particles
@@ -176,7 +176,9 @@ constexpr int kLeafCountShift = 27;
 
 // Per-warp shared staging.
 struct WalkSmem {
-  uint2 stack[kWalkStack];          // {first child | (count-1) << 29, lane mask}
+  // {first child | (count-1) << 29, lane mask}, above kWalkRanges empty entries (mask
+  // 0) that a round reads when fewer ranges are left
+  uint2 stack[kWalkRanges + kWalkStack];
   uint2 q[kLeafFlush + 32];         // opened leaves: {first | (count-1) << 27, opening mask}
   union {
     struct {
@@ -418,14 +420,19 @@ __device__ inline uint32_t set_gt_mask(float a, float b) {
 }
 
 // Transpose of the 32 x 32 bit matrix held one row per lane: afterwards bit j
-// of lane i is bit i of lane j (five butterfly stages of 16, 8, 4, 2, 1 bits).
+// of lane i is bit i of lane j (five butterfly stages of 16, 8, 4, 2, 1 bits). The
+// stages of 16 and 8 bits are one byte permutation each, the others a rotation and a
+// bit select.
 __device__ __forceinline__ uint32_t warp_transpose(uint32_t x, int lane) {
-  const uint32_t m16 = 0x0000FFFFu, m8 = 0x00FF00FFu, m4 = 0x0F0F0F0Fu, m2 = 0x33333333u, m1 = 0x55555555u;
+  x = __byte_perm(x, __shfl_xor_sync(0xffffffffu, x, 16), lane & 16 ? 0x3276 : 0x5410);
+  x = __byte_perm(x, __shfl_xor_sync(0xffffffffu, x, 8), lane & 8 ? 0x3715 : 0x6240);
 #pragma unroll
-  for (int j = 16; j >= 1; j >>= 1) {
-    const uint32_t m = j == 16 ? m16 : j == 8 ? m8 : j == 4 ? m4 : j == 2 ? m2 : m1;
+  for (int j = 4; j >= 1; j >>= 1) {
+    const uint32_t m = j == 4 ? 0x0F0F0F0Fu : j == 2 ? 0x33333333u : 0x55555555u;
     const uint32_t y = __shfl_xor_sync(0xffffffffu, x, j);
-    x = (lane & j) ? ((x & ~m) | ((y >> j) & m)) : ((x & m) | ((y & m) << j));
+    // the bits a rotation wraps around fall on the kept ones
+    const uint32_t keep = lane & j ? ~m : m, in = __funnelshift_l(y, y, lane & j ? 32 - j : j);
+    x = (x & keep) | (in & ~keep);
   }
   return x;
 }
@@ -439,7 +446,7 @@ __device__ __forceinline__ uint32_t warp_transpose(uint32_t x, int lane) {
 // LPP: lanes per particle (walk group of 32 / LPP particles); a launch walks the
 // galaxies whose SegDesc wlpp field equals LPP and skips the others' work items.
 template <bool SF, bool DBG, bool ONE, bool COMP, int LPP>
-__global__ void __launch_bounds__(kWalkThreads, kWalkResident) walk_kernel(WalkArgs a) {
+__global__ void __launch_bounds__(kWalkThreads, COMP ? kWalkResident - 1 : kWalkResident) walk_kernel(WalkArgs a) {
   static_assert(LPP == 1 || LPP == 2 || LPP == 4 || LPP == 8, "lanes per particle");
   constexpr uint32_t G = 32 / LPP;                         // particles per work item
   constexpr int NPP = 16 / LPP;                            // slot pairs a lane tests in a full round
@@ -461,6 +468,9 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkResident) walk_kernel(WalkA
   const uint32_t NS = ONE && LPP > 1 ? a.seg0.wsplit : 1u;
   const uint32_t nitems = a.L.groups * kStride * NS;
   const unsigned full = 0xffffffffu;
+
+  const uint32_t below = (1u << lane) - 1u, lanebit = 1u << pl;
+  if (lane < kWalkRanges) S.stack[lane] = make_uint2(0u, 0u);
 
   while (true) {
     uint32_t c = 0;  // grab the next work item of the schedule
@@ -490,15 +500,10 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkResident) walk_kernel(WalkA
     const uint32_t gbeg = sd.off + (gcur - sd.group0) * kWalkGroup + part * G, gend = gbeg + G;
     const uint32_t i = gbeg + pl;
     const bool valid = i < seg_end;
-    // Walk groups of 32 read the particle's record again for the integration at
-    // the end, so only its negated position stays live through the walk; smaller
-    // groups keep it (measured faster there).
-    constexpr bool kReload = LPP == 1;
+    // The particle's record is read again for the integration at the end, so only its
+    // negated position stays live through the walk.
     float4 p0 = make_float4(0.f, 0.f, 0.f, 0.f), p1 = p0;
-    if (valid) {
-      p0 = a.pin[2 * (size_t)i];
-      if (!kReload) p1 = a.pin[2 * (size_t)i + 1];
-    }
+    if (valid) p0 = a.pin[2 * (size_t)i];
     const float2 px = f2(-p0.x), py = f2(-p0.y), pz = f2(-p0.z);  // negated: r = q + (-p)
     Sums F = {f2(0.f), f2(0.f), f2(0.f), f2(0.f)};
     float2 cax = f2(0.f), cay = f2(0.f), caz = f2(0.f), cpt = f2(0.f);  // COMP only
@@ -530,7 +535,7 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkResident) walk_kernel(WalkA
     }
 
     int sp = 0;
-    if (lane == 0) S.stack[0] = make_uint2(sd.node_off, all);  // the root: range {node_off, 1}
+    if (lane == 0) S.stack[kWalkRanges] = make_uint2(sd.node_off, all);  // the root: range {node_off, 1}
     sp = idle ? 0 : 1;
     uint32_t budget = 4u * sd.node_cap + 1024u;
     while (true) {
@@ -542,11 +547,11 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkResident) walk_kernel(WalkA
       __syncwarp();
       // pop up to kWalkRanges ranges; their children are staged and tested together
       const int nr = min(sp, kWalkRanges);
-      const int sp0 = sp;
+      const uint2* const top = &S.stack[kWalkRanges + sp - 1];
       sp -= nr;
       uint32_t masks[kWalkRanges];  // lanes that opened each popped range's parent
 #pragma unroll
-      for (int r = 0; r < kWalkRanges; r++) masks[r] = r < nr ? S.stack[sp0 - 1 - r].y : 0u;
+      for (int r = 0; r < kWalkRanges; r++) masks[r] = top[-r].y;
       if (--budget == 0) {
         if (lane == 0) raise_err(sst, GS_DERR_STACK);
         break;
@@ -559,17 +564,16 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkResident) walk_kernel(WalkA
       uint32_t cnode = 0, cchild = 0, ccnt = 0;  // this lane's slot: node, first child or particle, count
       float csize = 1.f;
       if (lane < 8 * kWalkRanges) {
-        const int r = lane >> 3;
         const uint32_t c = lane & 7;
-        const uint2 e = r < nr ? S.stack[sp0 - 1 - r] : make_uint2(0u, 0u);
-        const uint32_t rs = e.x & 0x1fffffffu, rc = r < nr ? (e.x >> 29) + 1u : 0u;
+        const uint2 e = top[-(lane >> 3)];
+        const uint32_t rs = e.x & 0x1fffffffu;
         float4 q = make_float4(1e30f, 1e30f, 1e30f, 0.f);
         WalkInfo w;
         w.s2 = 0.f;
         w.child = 0;
         w.info = kLeafBit;
         w.size = 1.f;
-        bool real = c < rc, counted = true;
+        bool real = e.y != 0u && c <= e.x >> 29, counted = true;
         if (NS > 1 && real) {
           const uint32_t node = rs + c;
           if (node < up_end) counted = ksp == 0;                                    // levels above the split
@@ -609,19 +613,17 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkResident) walk_kernel(WalkA
       // per range: this lane active; the slots whose open bits this lane keeps (its
       // active ranges' eight slots: a slot past a range's count holds a dummy of
       // size^2 -inf, which every active lane accepts, so it never sets an open bit)
-      uint32_t actbits = 0, keep = 0;
-#pragma unroll
-      for (int r = 0; r < kWalkRanges; r++) {
-        const uint32_t a_r = (masks[r] >> pl) & 1u;
-        actbits |= a_r << r;
-        keep |= a_r ? 0xffu << (8 * r) : 0u;
-      }
-      keep &= mine;
       // theta^2 per range; a lane inactive for a range tests against -inf, so its
       // td is -inf (or NaN) and it accepts and adds nothing there
+      uint32_t act = 0;
       float th2[kWalkRanges];
 #pragma unroll
-      for (int r = 0; r < kWalkRanges; r++) th2[r] = (actbits >> r) & 1u ? theta2 : -INFINITY;
+      for (int r = 0; r < kWalkRanges; r++) {
+        const bool on = masks[r] & lanebit;
+        th2[r] = on ? theta2 : -INFINITY;
+        if (on) act |= 0xffu << (8 * r);
+      }
+      const uint32_t keep = act & mine;
       uint32_t obits = 0;  // children this lane opens (active, not accepted), bit = slot
       // COMP: the round's far-field terms (at most 32 per lane) are summed plainly,
       // then the round's sum joins the particle's total in one Kahan step
@@ -679,7 +681,7 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkResident) walk_kernel(WalkA
         const uint32_t cc = __ffs(bb) - 1;
         const uint32_t lf = __shfl_sync(full, cchild, cc), cnt = __shfl_sync(full, ccnt, cc);
         const float sz = __shfl_sync(full, csize, cc);
-        if (((actbits >> (cc >> 3)) & 1u) && (i - lf) < cnt) {
+        if (((act >> cc) & 1u) && (i - lf) < cnt) {
           dens = (float)cnt / (sz * sz * sz);
           // the leaf's direct sum includes the particle itself (softened walks)
           if (((obits & ~skipm) >> cc) & 1u) selfw += 1.0f;
@@ -696,44 +698,34 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkResident) walk_kernel(WalkA
       // mask to the stack, in slot order (prefix positions)
       const uint32_t pushc = om & ~leafmask;
       if (pushc) {
-        bool ok = false;
-        uint2 ent = make_uint2(0u, 0u);
-        if ((pushc >> lane) & 1u) {
-          // a galaxy's child ranges stay in its node range by construction (build,
-          // upload check); the walk itself only guards the pool bounds
-          ok = cchild > cnode && ccnt - 1u < 8u && cchild <= a.node_pool - ccnt;
-          if (!ok) raise_err(sst, GS_DERR_TREE);
-          ent = make_uint2(cchild | ((ccnt - 1u) << 29), col);
+        const int np = __popc(pushc);
+        if (sp + np > kWalkStack) {  // not for depth <= 10 trees
+          if (lane == 0) raise_err(sst, GS_DERR_STACK);
+        } else {
+          if ((pushc >> lane) & 1u) {
+            // a galaxy's child ranges stay in its node range by construction (build,
+            // upload check); the walk itself only guards the pool bounds
+            const bool ok = cchild > cnode && ccnt - 1u < 8u && cchild <= a.node_pool - ccnt;
+            if (!ok) raise_err(sst, GS_DERR_TREE);
+            S.stack[kWalkRanges + sp + __popc(pushc & below)] =
+                ok ? make_uint2(cchild | ((ccnt - 1u) << 29), col) : make_uint2(0u, 0u);
+          }
+          sp += np;
         }
-        const uint32_t okm = __ballot_sync(full, ok);
-        const int pos = sp + __popc(okm & ((1u << lane) - 1u));
-        if (ok && pos < kWalkStack) S.stack[pos] = ent;
-        const int np = __popc(okm);
-        if (sp + np > kWalkStack && lane == 0) raise_err(sst, GS_DERR_STACK);  // not for depth <= 10 trees
-        sp = min(sp + np, kWalkStack);
       }
       // Opened leaves: those of at most kLeafMax particles join the queue, in slot
       // order; larger ones (coincident particles at the deepest level) are summed
       // at once, in chunks of 32.
       const uint32_t leafc = om & leafmask & ~skipm;
       if (leafc) {
-        bool sm = false, bg = false;
-        uint2 ent = make_uint2(0u, 0u);
-        uint32_t np = 0;
-        if ((leafc >> lane) & 1u) {
-          if (ccnt > a.pool_n || cchild > a.pool_n - ccnt) {
-            raise_err(sst, GS_DERR_TREE);
-          } else {
-            bg = ccnt > kLeafMax;
-            sm = !bg && ccnt > 0u;  // an empty leaf adds nothing
-            ent = make_uint2(cchild | ((ccnt - 1u) << kLeafCountShift), col);
-            if (sm) np = (ccnt + 1u) >> 1;
-          }
-        }
-        const uint32_t smallm = __ballot_sync(full, sm);
-        if (sm) S.q[nq + __popc(smallm & ((1u << lane) - 1u))] = ent;
-        nq += __popc(smallm);
-        qp += __reduce_add_sync(full, np);
+        const bool mine_leaf = (leafc >> lane) & 1u;
+        // empty (adds nothing), large, or past the particle pool: not for the queue
+        const bool odd = mine_leaf && (ccnt - 1u >= kLeafMax || cchild > a.pool_n - ccnt);
+        const uint32_t oddm = __ballot_sync(full, odd), goodm = leafc & ~oddm;
+        const bool good = mine_leaf && !odd;
+        if (good) S.q[nq + __popc(goodm & below)] = make_uint2(cchild | ((ccnt - 1u) << kLeafCountShift), col);
+        nq += __popc(goodm);
+        qp += __reduce_add_sync(full, good ? (ccnt + 1u) >> 1 : 0u);
         if (DBG) {
           for (uint32_t bb = leafc; bb; bb &= bb - 1) {
             const uint32_t cc = __ffs(bb) - 1;
@@ -742,10 +734,14 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkResident) walk_kernel(WalkA
             if (sub == 0 && ((open >> pl) & 1u)) npair += cnt - (i - lf < cnt ? 1u : 0u);
           }
         }
-        for (uint32_t bb = __ballot_sync(full, bg); bb; bb &= bb - 1) {
+        for (uint32_t bb = oddm; bb; bb &= bb - 1) {
           const uint32_t cc = __ffs(bb) - 1;
           const unsigned open = __shfl_sync(full, col, cc);
           const uint32_t lf = __shfl_sync(full, cchild, cc), cnt = __shfl_sync(full, ccnt, cc);
+          if (cnt > a.pool_n || lf > a.pool_n - cnt) {
+            if (lane == 0) raise_err(sst, GS_DERR_TREE);
+            continue;
+          }
           for (uint32_t b0 = 0; b0 < cnt; b0 += 32) {
             const uint32_t k = min(32u, cnt - b0);
             __syncwarp();
@@ -841,7 +837,7 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkResident) walk_kernel(WalkA
         selfw = u2.y;
       }
     }
-    if (kReload && valid) {
+    if (valid) {
       p0 = a.pin[2 * (size_t)i];
       p1 = a.pin[2 * (size_t)i + 1];
     }
