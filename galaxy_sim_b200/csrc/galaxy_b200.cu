@@ -43,6 +43,7 @@ thread_local char g_err[512] = "";
 // host-side fault injection (gs_test_fail_alloc): the number of device
 // allocations still to succeed before one fails; negative: none fails
 std::atomic<long long> g_fail_alloc_in{-1};
+bool fail_this_alloc() { return g_fail_alloc_in.load() >= 0 && g_fail_alloc_in.fetch_sub(1) == 0; }
 
 constexpr uint64_t kMaxPool = 1ull << 27;  // node indices (2 cap + 4096) fit the walk's 29-bit fields
 constexpr uint32_t kMaxSlots = 4096;
@@ -112,6 +113,7 @@ uint64_t plan_bytes(const Plan& p) {
   b += (uint64_t)(p.sort_tiles + p.flag_tiles + p.groups) * 4;
   b += (uint64_t)p.groups * kWalkParts * kPartials * 8 + 16;
   b += (uint64_t)p.diag_chunks * kPartials * 8 + s * 4;
+  b += 40 * (256 + 16);  // alignment of the parts of the one allocation
   return b;
 }
 
@@ -290,7 +292,7 @@ struct gs_ctx {
   template <typename T>
   cudaError_t alloc(T** p, size_t count) {
     void* q = nullptr;
-    if (g_fail_alloc_in.load() >= 0 && g_fail_alloc_in.fetch_sub(1) == 0) return cudaErrorMemoryAllocation;
+    if (fail_this_alloc()) return cudaErrorMemoryAllocation;
     cudaError_t e = cudaMalloc(&q, count * sizeof(T) + 16);
     if (e != cudaSuccess) return e;
     owned.push_back(q);
@@ -403,7 +405,27 @@ int pool_init(gs_ctx* c, int device, uint64_t cap, uint32_t slots) {
   cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device);
   CK(c, cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking), "stream");
   CK(c, cudaEventCreateWithFlags(&c->ev, cudaEventDisableTiming), "event");
-#define A(ptr, cnt) CK(c, c->alloc(&(ptr), (cnt)), #ptr)
+  // One device allocation holds every buffer, those that start as zeros first: some 45
+  // cudaMallocs, frees and memsets cost 9.4 ms of a 14 ms sortAndBuild of 100000
+  // particles, which sets up a context for the call.
+  struct Part {
+    void** ptr;
+    size_t bytes;
+    const char* what;
+  };
+  std::vector<Part> zeroed, plain;
+#define Z(ptr, cnt) zeroed.push_back({reinterpret_cast<void**>(&(ptr)), sizeof(*(ptr)) * (size_t)(cnt) + 16, #ptr})
+#define A(ptr, cnt) plain.push_back({reinterpret_cast<void**>(&(ptr)), sizeof(*(ptr)) * (size_t)(cnt) + 16, #ptr})
+  Z(c->seg_ctr, p.slots);
+  Z(c->arrive, p.nodes);
+  Z(c->cm, p.nodes);
+  Z(c->info, p.nodes);
+  Z(c->meta, p.slots);
+  Z(c->st, p.slots);
+  Z(c->diag_out, (size_t)p.slots * kPartials);
+  Z(c->diag_ctr, p.slots);
+  Z(c->partials, (size_t)p.groups * kWalkParts * kPartials);
+  Z(c->walk_work, 4);
   A(c->part[0], 2 * p.cap);
   A(c->part[1], 2 * p.cap);
   A(c->stel[0], p.cap);
@@ -418,45 +440,42 @@ int pool_init(gs_ctx* c, int device, uint64_t cap, uint32_t slots) {
   A(c->vals[1], p.cap);
   A(c->sort_scratch, p.sort_words);
   A(c->bbox_part, (size_t)p.flag_tiles * 6);
-  A(c->seg_ctr, p.slots);
   A(c->frames, p.slots);
   A(c->dl, p.cap + 4);
   A(c->blk_counts, (size_t)p.flag_tiles * kCounters);
   A(c->blk_offs, (size_t)p.flag_tiles * kCounters);
-  A(c->meta, p.slots);
   A(c->node_start, p.nodes);
   A(c->child_base, p.nodes + 1);
   A(c->parent, p.nodes);
   A(c->depth, p.nodes);
-  A(c->arrive, p.nodes);
   A(c->leaf_node, p.cap + 1);
   A(c->leaf_start, p.cap + 1);
-  A(c->cm, p.nodes);
-  A(c->info, p.nodes);
-  A(c->st, p.slots);
-  A(c->diag_out, (size_t)p.slots * kPartials);
   A(c->diag_chunk, (size_t)p.diag_chunks * kPartials);
-  A(c->diag_ctr, p.slots);
   A(c->segs, p.slots);
   A(c->sort_map, p.sort_tiles);
   A(c->flag_map, p.flag_tiles);
   A(c->group_map, p.groups);
-  A(c->partials, (size_t)p.groups * kWalkParts * kPartials);
-  A(c->walk_work, 4);
 #undef A
-  CK(c, cudaMemset(c->seg_ctr, 0, sizeof(unsigned) * p.slots), "memset");
-  CK(c, cudaMemset(c->arrive, 0, sizeof(uint32_t) * p.nodes), "memset");
-  CK(c, cudaMemset(c->cm, 0, sizeof(float4) * p.nodes), "memset");
-  CK(c, cudaMemset(c->info, 0, sizeof(WalkInfo) * p.nodes), "memset");
-  CK(c, cudaMemset(c->meta, 0, sizeof(TreeMeta) * p.slots), "memset");
-  CK(c, cudaMemset(c->st, 0, sizeof(DevState) * p.slots), "memset");
-  CK(c, cudaMemset(c->diag_out, 0, sizeof(double) * kPartials * p.slots), "memset");
-  CK(c, cudaMemset(c->diag_ctr, 0, sizeof(unsigned) * p.slots), "memset");
-  CK(c, cudaMemset(c->partials, 0, sizeof(double) * kPartials * kWalkParts * p.groups), "memset");
-  CK(c, cudaMemset(c->walk_work, 0, 16), "memset");
-  CK(c, cudaMallocHost(&c->host_stage, sizeof(gs_params) * (size_t)gs_ctx::kParamRing + 256), "pinned stage");
-  for (int k = 0; k < gs_ctx::kParamRing; k++)
-    CK(c, cudaEventCreateWithFlags(&c->param_ev[k], cudaEventDisableTiming), "params event");
+#undef Z
+  size_t total = 0, zeros = 0;
+  for (const std::vector<Part>* v : {&zeroed, &plain}) {
+    for (const Part& q : *v) {
+      if (fail_this_alloc()) CK(c, cudaErrorMemoryAllocation, q.what);
+      total += (q.bytes + 255) / 256 * 256;
+    }
+    if (v == &zeroed) zeros = total;
+  }
+  char* arena = nullptr;
+  CK(c, cudaMalloc(reinterpret_cast<void**>(&arena), total), "pool buffers");
+  c->owned.push_back(arena);
+  char* at = arena;
+  for (const std::vector<Part>* v : {&zeroed, &plain})
+    for (const Part& q : *v) {
+      *q.ptr = at;
+      at += (q.bytes + 255) / 256 * 256;
+    }
+  CK(c, cudaMemsetAsync(arena, 0, zeros, c->stream), "memset");
+  CK(c, cudaStreamSynchronize(c->stream), "memset");
   c->slots.assign(p.slots, Slot());
   c->palloc.init(p.cap);
   c->lay_dirty = true;
@@ -951,6 +970,44 @@ int host_pack4(const float* src, uint32_t N, uint32_t stride, std::vector<float4
   return GS_OK;
 }
 
+int params_stage(gs_ctx* c) {
+  CK(c, cudaMallocHost(&c->host_stage, sizeof(gs_params) * (size_t)gs_ctx::kParamRing + 256), "pinned stage");
+  for (int k = 0; k < gs_ctx::kParamRing; k++)
+    CK(c, cudaEventCreateWithFlags(&c->param_ev[k], cudaEventDisableTiming), "params event");
+  return GS_OK;
+}
+
+// params: set up the staging of Params uploads (the stateless calls' contexts take none).
+int pool_create(int device, uint64_t particle_capacity, uint32_t max_galaxies, bool params, gs_ctx** out) {
+  if (!out) {
+    set_err(g_err, "out is NULL");
+    return GS_EINVAL;
+  }
+  *out = nullptr;
+  if (particle_capacity == 0 || particle_capacity > kMaxPool || max_galaxies == 0 ||
+      max_galaxies > kMaxSlots) {
+    set_err(g_err, "pool capacity must be in [1, %llu] particles and [1, %u] galaxies",
+            (unsigned long long)kMaxPool, kMaxSlots);
+    return GS_EINVAL;
+  }
+  int ndev = 0;
+  if (cudaGetDeviceCount(&ndev) != cudaSuccess || device < 0 || device >= ndev) {
+    set_err(g_err, "no CUDA device %d (have %d)", device, ndev);
+    return GS_EINVAL;
+  }
+  gs_ctx* c = new (std::nothrow) gs_ctx();
+  if (!c) return GS_ENOMEM;
+  int rc = pool_init(c, device, particle_capacity, max_galaxies);
+  if (!rc && params) rc = params_stage(c);
+  if (rc) {
+    set_err(g_err, "%s", c->err);
+    gs_destroy(c);
+    return rc;
+  }
+  *out = c;
+  return GS_OK;
+}
+
 }  // namespace
 
 // Context-free error text for entry points defined in other translation units.
@@ -996,32 +1053,7 @@ uint64_t gs_pool_bytes(uint64_t particle_capacity, uint32_t max_galaxies) {
 }
 
 int gs_pool_create(int device, uint64_t particle_capacity, uint32_t max_galaxies, gs_ctx** out) {
-  if (!out) {
-    set_err(g_err, "out is NULL");
-    return GS_EINVAL;
-  }
-  *out = nullptr;
-  if (particle_capacity == 0 || particle_capacity > kMaxPool || max_galaxies == 0 ||
-      max_galaxies > kMaxSlots) {
-    set_err(g_err, "pool capacity must be in [1, %llu] particles and [1, %u] galaxies",
-            (unsigned long long)kMaxPool, kMaxSlots);
-    return GS_EINVAL;
-  }
-  int ndev = 0;
-  if (cudaGetDeviceCount(&ndev) != cudaSuccess || device < 0 || device >= ndev) {
-    set_err(g_err, "no CUDA device %d (have %d)", device, ndev);
-    return GS_EINVAL;
-  }
-  gs_ctx* c = new (std::nothrow) gs_ctx();
-  if (!c) return GS_ENOMEM;
-  const int rc = pool_init(c, device, particle_capacity, max_galaxies);
-  if (rc) {
-    set_err(g_err, "%s", c->err);
-    gs_destroy(c);
-    return rc;
-  }
-  *out = c;
-  return GS_OK;
+  return pool_create(device, particle_capacity, max_galaxies, true, out);
 }
 
 int gs_pool_add(gs_ctx* ctx, uint32_t N, const float* particles8, const float* stellar4,
@@ -1771,7 +1803,7 @@ struct TmpCtx {
 int tmp_init(TmpCtx& t, uint32_t N, uint32_t max_nodes) {
   int dev = 0;
   cudaGetDevice(&dev);
-  int rc = gs_pool_create(dev, N, 1, &t.c);
+  int rc = pool_create(dev, N, 1, false, &t.c);
   if (rc) return rc;
   gs_ctx* c = t.c;
   Slot& s = c->slots[0];
@@ -1873,6 +1905,11 @@ int tree_outputs(TmpCtx& t, uint32_t max_nodes, gs_node* nodes, uint32_t* num_no
 // Failure-detection settings of the two radix-sort entry points (gs_test_sort_lookback).
 std::atomic<uint32_t> g_test_spin_limit{kSpinLimit};
 std::atomic<uint32_t> g_test_withhold{kNoTile};
+
+__global__ void masses_kernel(const float4* __restrict__ P, float* __restrict__ out, uint32_t N) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x)
+    out[i] = P[2 * (size_t)i].w;
+}
 
 __global__ void mask30_kernel(uint32_t* keys, uint32_t N) {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x)
@@ -2030,8 +2067,14 @@ int gs_sort_and_build(const float* particles8, const float* stellar4, uint32_t N
   gather_kernel<<<c->lay.flag_tiles, kTileThreads, 0, c->stream>>>(c->vals[0], P, P2, S, S2, c->lay, c->st);
   enqueue_build(c, P2, 2, kComJs, 0.0, c->frames);
   TK(cudaGetLastError(), "sort and build");
-  std::vector<uint32_t> hp(N);
-  TK(cudaMemcpyAsync(hp.data(), c->vals[0], sizeof(uint32_t) * N, cudaMemcpyDeviceToHost, c->stream), "perm");
+  std::vector<uint32_t> hp(perm ? 0 : N);
+  uint32_t* const pm = perm ? perm : hp.data();
+  TK(cudaMemcpyAsync(pm, c->vals[0], sizeof(uint32_t) * N, cudaMemcpyDeviceToHost, c->stream), "perm");
+  if (sorted_mass) {  // one word of each record, packed on the device
+    masses_kernel<<<grid_for(N, 256, 148 * 8), 256, 0, c->stream>>>(P2, c->energy, N);
+    TK(cudaGetLastError(), "masses");
+    TK(cudaMemcpyAsync(sorted_mass, c->energy, sizeof(float) * N, cudaMemcpyDeviceToHost, c->stream), "masses");
+  }
   if (sorted8) TK(cudaMemcpyAsync(sorted8, P2, (size_t)N * 32, cudaMemcpyDeviceToHost, c->stream), "sorted");
   if (sorted_stellar4)
     TK(cudaMemcpyAsync(sorted_stellar4, S2, (size_t)N * 16, cudaMemcpyDeviceToHost, c->stream), "stellar");
@@ -2039,17 +2082,11 @@ int gs_sort_and_build(const float* particles8, const float* stellar4, uint32_t N
   if (rc) return rc;
   int64_t c1 = 0, c2 = -1;
   for (uint32_t i = 0; i < N; i++) {
-    if (hp[i] == 0) c1 = i;
-    if ((int64_t)hp[i] == track_idx2) c2 = i;
+    if (pm[i] == 0) c1 = i;
+    if ((int64_t)pm[i] == track_idx2) c2 = i;
   }
-  if (perm) memcpy(perm, hp.data(), sizeof(uint32_t) * N);
   if (central_idx) *central_idx = c1;
   if (central_idx2) *central_idx2 = c2;
-  if (sorted_mass) {
-    std::vector<float> s8((size_t)N * 8);
-    TK(cudaMemcpy(s8.data(), P2, (size_t)N * 32, cudaMemcpyDeviceToHost), "mass");
-    for (uint32_t i = 0; i < N; i++) sorted_mass[i] = s8[(size_t)i * 8 + 3];
-  }
   return GS_OK;
 }
 
