@@ -248,6 +248,7 @@ struct gs_ctx {
   int walk_group = 32;             // tuning: walk group size (0: by galaxy size; 4, 8, 16 or 32 particles)
   int walk_split = 1;              // tuning: walk splits per work item of a lone galaxy (0: by its size; 1, 2, 4, 8)
   uint32_t walk_items[4] = {0, 0, 0, 0};  // work items per lanes-per-particle class (1, 2, 4, 8)
+  bool cluster_ok = false; // the device runs a refresh's level loop on one cluster
   bool fuse_ok = false;    // the layout's galaxy is rebuilt by one kernel on one cluster
   bool walk_comp = false;  // compensated far-field sums in the walk (a Kahan step per round)
   // pinned staging of Params uploads: a ring of entries, each rewritten only after
@@ -397,6 +398,37 @@ bool fuse_supported(uint32_t n) {
   return true;
 }
 
+void refresh_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute attr[2], cudaStream_t s) {
+  cfg = {};
+  cfg.gridDim = dim3(kFuseCtas);
+  cfg.blockDim = dim3(kRefreshThreads);
+  cfg.stream = s;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = kFuseCtas;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+}
+
+// Whether the current device runs the level loop of a refresh on one cluster.
+bool refresh_supported() {
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attr[2];
+  refresh_config(cfg, attr, nullptr);
+  cfg.numAttrs = 1;  // the cluster shape
+  int clusters = 0;
+  cudaError_t e =
+      cudaFuncSetAttribute((const void*)refresh_internal_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&clusters, (const void*)refresh_internal_kernel, &cfg);
+  if (e != cudaSuccess || clusters < 1) {
+    cudaGetLastError();  // a refresh then launches once per level
+    return false;
+  }
+  return true;
+}
+
 int pool_init(gs_ctx* c, int device, uint64_t cap, uint32_t slots) {
   c->device = device;
   c->plan = make_plan(cap, slots);
@@ -476,6 +508,7 @@ int pool_init(gs_ctx* c, int device, uint64_t cap, uint32_t slots) {
     }
   CK(c, cudaMemsetAsync(arena, 0, zeros, c->stream), "memset");
   CK(c, cudaStreamSynchronize(c->stream), "memset");
+  c->cluster_ok = refresh_supported();
   c->slots.assign(p.slots, Slot());
   c->palloc.init(p.cap);
   c->lay_dirty = true;
@@ -1308,14 +1341,40 @@ int gs_refresh(gs_ctx* ctx) {
     if (s.tree == Slot::kTreeBuilt) built = true;
     if (s.tree != Slot::kTreeUploaded) continue;
     // NBodyGPU.js:309: no-op without levelRanges; deepest level first
-    for (int64_t l = (int64_t)s.up_lr.size() / 2 - 1; l >= 0; l--) {
+    const int64_t nl = (int64_t)s.up_lr.size() / 2;
+    RefreshLevels lv;
+    lv.n = (uint32_t)nl;
+    bool in_order = nl > 0;  // the levels follow one another, as MortonTree.build numbers them
+    uint32_t next = nl ? s.up_lr[0] : 0u;
+    const uint32_t first = next;
+    for (int64_t l = nl - 1; l >= 0; l--) {
       const uint32_t start = s.up_lr[2 * l], count = s.up_lr[2 * l + 1];
-      if (!count) continue;
-      if ((uint64_t)start + count > s.up_nodes)
+      if (count && (uint64_t)start + count > s.up_nodes)
         return ctx->fail(GS_EINVAL, "level %lld [%u, +%u) beyond %u nodes", (long long)l, start, count,
                          s.up_nodes);
-      refresh_level_kernel<<<cdiv(count, 64), 64, 0, ctx->stream>>>(ctx->part[ctx->cur], ctx->cm, ctx->info,
-                                                                     s.node_off + start, count);
+    }
+    for (int64_t l = 0; l < nl && in_order; l++) {
+      in_order = s.up_lr[2 * l] == next;
+      lv.start[l] = s.node_off + next;
+      lv.count[l] = s.up_lr[2 * l + 1];
+      next += lv.count[l];
+    }
+    if (in_order && ctx->cluster_ok) {
+      if (next == first) continue;  // levels without nodes
+      launch_pdl(refresh_leaves_kernel, cdiv(next - first, 256), 256, ctx->stream,
+                 (const float4*)ctx->part[ctx->cur], ctx->cm, (const WalkInfo*)ctx->info, s.node_off + first,
+                 next - first);
+      cudaLaunchConfig_t cfg;
+      cudaLaunchAttribute attr[2];
+      refresh_config(cfg, attr, ctx->stream);
+      cudaLaunchKernelEx(&cfg, refresh_internal_kernel, ctx->cm, (const WalkInfo*)ctx->info, lv);
+      continue;
+    }
+    for (int64_t l = nl - 1; l >= 0; l--) {
+      const uint32_t start = s.up_lr[2 * l], count = s.up_lr[2 * l + 1];
+      if (count)
+        refresh_level_kernel<<<cdiv(count, 64), 64, 0, ctx->stream>>>(ctx->part[ctx->cur], ctx->cm, ctx->info,
+                                                                       s.node_off + start, count);
     }
   }
   if (built && ctx->lay.nseg) {

@@ -6,6 +6,8 @@
 // The per-particle kernels run one 1024-particle tile per block over the tile
 // list of a batch layout; a tile lies inside one galaxy.
 #pragma once
+#include <cooperative_groups.h>
+
 #include "build.cuh"
 #include "common.cuh"
 #include "morton.cuh"
@@ -326,6 +328,64 @@ __global__ void refresh_level_kernel(const float4* __restrict__ P, float4* cm,
     }
   }
   cm[n] = m > 0.0f ? make_float4(cx / m, cy / m, cz / m, m) : make_float4(0.f, 0.f, 0.f, m);
+}
+
+// refresh_level over a whole uploaded tree whose level ranges follow one another
+// (every MortonTree.build output): the leaves of all levels at once on the full grid,
+// then the internal nodes level by level, deepest first, on one cluster with a barrier per
+// level. Sums and results are refresh_level_kernel's.
+//
+// What bounds it: latency. A tree of 100000 particles has ten levels; as one launch each
+// they took 3.5 to 10 us (a leaf's particles were loaded one after another, 16 round
+// trips). Refresh and step of that tree: 328 us with one launch per level, 283 so.
+__global__ void __launch_bounds__(256)
+    refresh_leaves_kernel(const float4* __restrict__ P, float4* cm, const WalkInfo* __restrict__ info,
+                          uint32_t start, uint32_t count) {
+  griddep_wait();  // launched with a programmatic dependency: predecessors' writes first
+  const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= count) return;
+  const WalkInfo w = info[start + g];
+  if (!(w.info & kLeafBit)) return;
+  const uint32_t cnt = w.info & ~kLeafBit;
+  ComSum<false> sum;
+  for (uint32_t j0 = 0; j0 < cnt; j0 += kComChunk) {
+    float4 q[kComChunk];
+#pragma unroll
+    for (uint32_t k = 0; k < kComChunk; k++) q[k] = P[2 * (size_t)(w.child + min(j0 + k, cnt - 1))];
+#pragma unroll
+    for (uint32_t k = 0; k < kComChunk; k++)
+      if (j0 + k < cnt) sum.add(q[k]);
+  }
+  cm[start + g] = sum.mean();
+}
+
+constexpr int kRefreshThreads = 512;
+struct RefreshLevels {
+  uint32_t n, start[16], count[16];  // pool indices of the levels, root first
+};
+__global__ void __launch_bounds__(kRefreshThreads)
+    refresh_internal_kernel(float4* cm, const WalkInfo* __restrict__ info, RefreshLevels lv) {
+  namespace cg = cooperative_groups;
+  griddep_wait();  // launched with a programmatic dependency: predecessors' writes first
+  cg::cluster_group cl = cg::this_cluster();
+  const uint32_t t = cl.block_rank() * kRefreshThreads + threadIdx.x, T = cl.num_blocks() * kRefreshThreads;
+  for (int l = (int)lv.n - 1; l >= 0; l--) {
+    for (uint32_t g = t; g < lv.count[l]; g += T) {
+      const uint32_t n = lv.start[l] + g;
+      const WalkInfo w = info[n];
+      if (w.info & kLeafBit) continue;
+      float4 q[8];
+#pragma unroll
+      for (uint32_t k = 0; k < 8; k++)
+        q[k] = k < w.info ? __ldcg(&cm[w.child + k]) : make_float4(0.f, 0.f, 0.f, 0.f);
+      ComSum<false> sum;
+#pragma unroll
+      for (uint32_t k = 0; k < 8; k++)
+        if (k < w.info) sum.add(q[k]);
+      cm[n] = sum.mean();
+    }
+    cl.sync();
+  }
 }
 
 // uploadBHTree: BHNode (64 B) -> walk layout of one galaxy, whose nodes start at
