@@ -623,13 +623,13 @@ int ensure_layout(gs_ctx* c) {
     if (arr > c->split_arrive_cap) {
       unsigned* p = nullptr;
       CK(c, c->alloc(&p, arr), "split walk arrivals");
-      CK(c, cudaMemset(p, 0, arr * sizeof(unsigned)), "memset");
+      CK(c, cudaMemsetAsync(p, 0, arr * sizeof(unsigned), c->stream), "memset");
       c->split_arrive = p;
       c->split_arrive_cap = arr;
     }
   }
   if (!h.empty()) {
-    CK(c, cudaMemcpy(c->segs, h.data(), sizeof(SegDesc) * h.size(), cudaMemcpyHostToDevice), "layout");
+    CK(c, cudaMemcpyAsync(c->segs, h.data(), sizeof(SegDesc) * h.size(), cudaMemcpyHostToDevice, c->stream), "layout");
     const uint32_t tot = std::max(st, std::max(ft, gr));
     layout_maps_kernel<<<grid_for(tot, 256, 148 * 8), 256, 0, c->stream>>>(
         c->segs, (uint32_t)h.size(), c->sort_map, st, c->flag_map, ft, c->group_map, gr);
@@ -948,29 +948,33 @@ int stage_grow(gs_ctx* c, uint32_t need_nodes) {
 }
 
 // Put a galaxy into slot `slot` at pool offset off (both ping-pongs written).
+// Uploads and fills run on the context's stream, which does not wait for the default stream: a
+// plain cudaMemcpy from pageable memory may return with its last piece under way there,
+// and a kernel on this stream could read ahead of it.
 int slot_fill(gs_ctx* c, uint32_t slot, uint32_t off, uint32_t span, uint32_t n, uint32_t node_cap,
               const float* particles8, const float* stellar4, const gs_params* params) {
   Slot& s = c->slots[slot];
   CK(c, cudaStreamSynchronize(c->stream), "sync");
   const size_t pb = (size_t)n * 32, sb = (size_t)n * 16;
   for (int k = 0; k < 2; k++) {
-    CK(c, cudaMemcpy(c->part[k] + 2 * (size_t)off, particles8, pb, cudaMemcpyHostToDevice), "upload");
+    CK(c, cudaMemcpyAsync(c->part[k] + 2 * (size_t)off, particles8, pb, cudaMemcpyHostToDevice, c->stream), "upload");
     if (stellar4)
-      CK(c, cudaMemcpy(c->stel[k] + off, stellar4, sb, cudaMemcpyHostToDevice), "upload");
+      CK(c, cudaMemcpyAsync(c->stel[k] + off, stellar4, sb, cudaMemcpyHostToDevice, c->stream), "upload");
     else
-      CK(c, cudaMemset(c->stel[k] + off, 0, sb), "memset");
+      CK(c, cudaMemsetAsync(c->stel[k] + off, 0, sb, c->stream), "memset");
   }
-  CK(c, cudaMemset(c->cm + 2 * (size_t)off, 0, sizeof(float4) * node_cap), "memset");
-  CK(c, cudaMemset(c->info + 2 * (size_t)off, 0, sizeof(WalkInfo) * node_cap), "memset");
-  CK(c, cudaMemset(c->meta + slot, 0, sizeof(TreeMeta)), "memset");
-  CK(c, cudaMemset(c->diag_out + (size_t)slot * kPartials, 0, sizeof(double) * kPartials), "memset");
+  CK(c, cudaMemsetAsync(c->cm + 2 * (size_t)off, 0, sizeof(float4) * node_cap, c->stream), "memset");
+  CK(c, cudaMemsetAsync(c->info + 2 * (size_t)off, 0, sizeof(WalkInfo) * node_cap, c->stream), "memset");
+  CK(c, cudaMemsetAsync(c->meta + slot, 0, sizeof(TreeMeta), c->stream), "memset");
+  CK(c, cudaMemsetAsync(c->diag_out + (size_t)slot * kPartials, 0, sizeof(double) * kPartials, c->stream), "memset");
   DevState st0;
   memset(&st0, 0, sizeof(st0));
   if (params) st0.p = *params;
   st0.p.N = n;
   st0.sim_time = (double)st0.p.time;
   st0.central[0] = st0.central[1] = -1;
-  CK(c, cudaMemcpy(c->st + slot, &st0, sizeof(st0), cudaMemcpyHostToDevice), "state");
+  CK(c, cudaMemcpyAsync(c->st + slot, &st0, sizeof(st0), cudaMemcpyHostToDevice, c->stream), "state");
+  CK(c, cudaStreamSynchronize(c->stream), "sync");  // the caller's arrays are free on return
   s = Slot();
   s.live = true;
   s.off = off;
@@ -1210,7 +1214,8 @@ int gs_set_time(gs_ctx* ctx, double t) {
   SLOT(ctx, s);
   (void)s;
   CK(ctx, cudaStreamSynchronize(ctx->stream), "sync");
-  CK(ctx, cudaMemcpy(&ctx->st[ctx->sel].sim_time, &t, sizeof(double), cudaMemcpyHostToDevice), "time");
+  CK(ctx, cudaMemcpyAsync(&ctx->st[ctx->sel].sim_time, &t, sizeof(double), cudaMemcpyHostToDevice, ctx->stream), "time");
+  CK(ctx, cudaStreamSynchronize(ctx->stream), "sync");
   return GS_OK;
 }
 
@@ -1220,7 +1225,8 @@ int gs_set_star_formation(gs_ctx* ctx, int enable) {
   (void)s;
   CK(ctx, cudaStreamSynchronize(ctx->stream), "sync");
   const unsigned off = enable ? 0u : 1u;
-  CK(ctx, cudaMemcpy(&ctx->st[ctx->sel].sf_off, &off, sizeof(off), cudaMemcpyHostToDevice), "sf flag");
+  CK(ctx, cudaMemcpyAsync(&ctx->st[ctx->sel].sf_off, &off, sizeof(off), cudaMemcpyHostToDevice, ctx->stream), "sf flag");
+  CK(ctx, cudaStreamSynchronize(ctx->stream), "sync");
   return GS_OK;
 }
 
@@ -1230,9 +1236,10 @@ int gs_update_central_mass(gs_ctx* ctx, float mass, uint32_t idx) {
   if (idx >= s->n) return ctx->fail(GS_EINVAL, "central index %u >= N %u", idx, s->n);
   CK(ctx, cudaStreamSynchronize(ctx->stream), "sync");
   for (int k = 0; k < 2; k++)
-    CK(ctx, cudaMemcpy(reinterpret_cast<char*>(ctx->part[k]) + ((size_t)s->off + idx) * 32 + 12, &mass, 4,
-                       cudaMemcpyHostToDevice),
+    CK(ctx, cudaMemcpyAsync(reinterpret_cast<char*>(ctx->part[k]) + ((size_t)s->off + idx) * 32 + 12, &mass, 4,
+                            cudaMemcpyHostToDevice, ctx->stream),
        "central mass");
+  CK(ctx, cudaStreamSynchronize(ctx->stream), "sync");
   return GS_OK;
 }
 
@@ -1280,7 +1287,9 @@ int gs_upload_tree(gs_ctx* ctx, const gs_node* nodes, uint32_t num_nodes,
   int rc = stage_grow(ctx, n);
   if (rc) return rc;
   CK(ctx, cudaStreamSynchronize(ctx->stream), "sync");
-  if (n) CK(ctx, cudaMemcpy(ctx->bh, nodes, (size_t)n * sizeof(gs_node), cudaMemcpyHostToDevice), "tree");
+  // on this stream: a plain cudaMemcpy's last piece may land after the kernel below starts
+  if (n)
+    CK(ctx, cudaMemcpyAsync(ctx->bh, nodes, (size_t)n * sizeof(gs_node), cudaMemcpyHostToDevice, ctx->stream), "tree");
   // the build's leaves pass skips this galaxy until its next on-device build
   CK(ctx, cudaMemsetAsync(ctx->meta + ctx->sel, 0, sizeof(TreeMeta), ctx->stream), "meta");
   if (n)
@@ -1794,7 +1803,7 @@ int gs_device_errors(gs_ctx* ctx, uint32_t* bits, int clear) {
   unsigned e = 0;
   CK(ctx, cudaMemcpy(&e, &ctx->st[ctx->sel].err, 4, cudaMemcpyDeviceToHost), "err");
   if (bits) *bits = e;
-  if (clear) CK(ctx, cudaMemset(&ctx->st[ctx->sel].err, 0, 4), "clear");
+  if (clear) CK(ctx, cudaMemsetAsync(&ctx->st[ctx->sel].err, 0, 4, ctx->stream), "clear");
   return GS_OK;
 }
 
@@ -1807,7 +1816,7 @@ int gs_counters(gs_ctx* ctx, uint64_t out[3], int reset) {
   CK(ctx, cudaMemcpy(c, ctx->st[ctx->sel].counters, sizeof(c), cudaMemcpyDeviceToHost), "counters");
   if (out)
     for (int k = 0; k < 3; k++) out[k] = c[k];
-  if (reset) CK(ctx, cudaMemset(ctx->st[ctx->sel].counters, 0, sizeof(c)), "reset");
+  if (reset) CK(ctx, cudaMemsetAsync(ctx->st[ctx->sel].counters, 0, sizeof(c), ctx->stream), "reset");
   return GS_OK;
 }
 
@@ -1840,7 +1849,7 @@ int tmp_init(TmpCtx& t, uint32_t N, uint32_t max_nodes) {
   DevState st0;
   memset(&st0, 0, sizeof(st0));
   st0.central[0] = st0.central[1] = -1;
-  if (cudaMemcpy(c->st, &st0, sizeof(st0), cudaMemcpyHostToDevice) != cudaSuccess) {
+  if (cudaMemcpyAsync(c->st, &st0, sizeof(st0), cudaMemcpyHostToDevice, c->stream) != cudaSuccess) {
     set_err(g_err, "state upload failed");
     return GS_ECUDA;
   }
