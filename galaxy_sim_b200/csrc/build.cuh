@@ -34,6 +34,7 @@ constexpr int kFlagThreads = 256;
 constexpr int kFlagPer = 4;                          // consecutive particles per thread
 constexpr int kFlagTile = kFlagThreads * kFlagPer;   // 1024 particles per block
 constexpr int kCounters = 12;                        // depths 0..10 + leaf starts
+constexpr int kTileWords = kCounters + 1;            // a tile's counts, then its depth masks
 
 // cpd of two codes: leading equal 3-bit digits (0..10).
 __device__ inline int cpd(uint32_t a, uint32_t b) {
@@ -46,8 +47,12 @@ __device__ inline int cpd(uint32_t a, uint32_t b) {
 struct BuildBuffers {
   const uint32_t* codes;  // sorted codes [pool]
   uint8_t* dl;            // packed D | L << 4 per particle [pool]
-  uint32_t* blk_counts;   // [flag tiles][12]
-  uint32_t* blk_offs;     // [flag tiles][12]
+  // [flag tiles][kTileWords]: node starts per depth and leaf starts; then a word of depth
+  // masks: bit d = some start with D <= d, bit 16 + d = the last of them has L > d
+  uint32_t* blk_counts;
+  // [flag tiles][kTileWords]: starts before the tile; then the depths (bit d) at which an
+  // internal node of an earlier tile is open where the tile begins
+  uint32_t* blk_offs;
   TreeMeta* meta;         // [slots]
   uint32_t* node_start;   // [node pool] first particle of the node
   uint32_t* child_base;   // [node pool]
@@ -60,13 +65,14 @@ struct BuildBuffers {
   WalkInfo* info;         // [node pool]
 };
 
-// K1: per particle D, L and per-tile start counts.
-__global__ void __launch_bounds__(kFlagThreads) tree_flags_kernel(BuildBuffers b, Layout Lo) {
-  griddep_wait();  // launched with a programmatic dependency: predecessors' writes first
+// Per particle D, L; per-tile start counts and depth masks.
+__device__ __forceinline__ void tile_flags(const BuildBuffers& b, const Layout& Lo) {
   __shared__ uint32_t s_code[kFlagTile + 32];
   __shared__ int8_t s_cpd16[kFlagTile + 16];
   __shared__ uint32_t s_red[kFlagThreads / 32][kCounters];
+  __shared__ uint32_t s_last[kDepths];  // last start with D <= d: (slot + 1) << 1 | (L > d)
   const int tid = threadIdx.x;
+  if (tid < kDepths) s_last[tid] = 0u;
   const uint32_t tile = blockIdx.x;
   const SegDesc sd = Lo.segs[Lo.seg_of_flag_tile[tile]];
   const int64_t seg_beg = sd.off, seg_end = (int64_t)sd.off + sd.n;
@@ -124,12 +130,42 @@ __global__ void __launch_bounds__(kFlagThreads) tree_flags_kernel(BuildBuffers b
     const uint32_t v = __reduce_add_sync(0xffffffffu, cnt[k]);
     if (lane == 0) s_red[warp][k] = v;
   }
+#pragma unroll
+  for (int d = 0; d < kDepths; d++) {
+    uint32_t v = 0;
+#pragma unroll
+    for (int q = 0; q < kFlagPer; q++) {
+      const int D = (packed >> (8 * q)) & 15, L = (packed >> (8 * q + 4)) & 15;
+      if (base + tid * kFlagPer + q < seg_end && D <= L && D <= d)
+        v = (uint32_t)(tid * kFlagPer + q + 1) << 1 | (L > d ? 1u : 0u);
+    }
+    v = __reduce_max_sync(0xffffffffu, v);
+    if (lane == 0 && v) atomicMax(&s_last[d], v);
+  }
   __syncthreads();
   if (tid < kCounters) {
     uint32_t s = 0;
     for (int w = 0; w < kFlagThreads / 32; w++) s += s_red[w][tid];
-    b.blk_counts[(size_t)tile * kCounters + tid] = s;
+    b.blk_counts[(size_t)tile * kTileWords + tid] = s;
   }
+  if (warp == 1) {
+    const uint32_t v = lane < kDepths ? s_last[lane] : 0u;
+    const uint32_t has = __ballot_sync(0xffffffffu, v != 0u), open = __ballot_sync(0xffffffffu, v & 1u);
+    if (lane == 0) b.blk_counts[(size_t)tile * kTileWords + kCounters] = has | open << 16;
+  }
+}
+
+// K1 of the stateless builds (a rebuild on the device runs it with the gather).
+__global__ void __launch_bounds__(kFlagThreads) tree_flags_kernel(BuildBuffers b, Layout Lo) {
+  griddep_wait();  // launched with a programmatic dependency: predecessors' writes first
+  tile_flags(b, Lo);
+}
+
+// Depth masks of two runs of tiles side by side: a depth's state is the later run's
+// where that has a start of it.
+__device__ __forceinline__ uint32_t join_masks(uint32_t a, uint32_t b) {
+  const uint32_t bh = b & 0xffffu;
+  return (a & 0xffffu) | bh | (((a >> 16) & ~bh) | (b >> 16)) << 16;
 }
 
 // K2: one block per galaxy scans its tiles' counts and fills its TreeMeta.
@@ -141,6 +177,7 @@ __global__ void __launch_bounds__(kScanThreads)
   griddep_wait();  // launched with a programmatic dependency: predecessors' writes first
   __shared__ uint32_t s_warp[kScanThreads / 32][kCounters];
   __shared__ uint32_t s_tot[kCounters];
+  __shared__ uint32_t s_mask[kScanThreads / 32];
   const uint32_t seg = blockIdx.x;
   const SegDesc sd = Lo.segs[seg];
   const uint32_t t0 = sd.flag_tile0, ntiles = (sd.n + kFlagTile - 1) / kFlagTile;
@@ -150,9 +187,21 @@ __global__ void __launch_bounds__(kScanThreads)
   uint32_t sum[kCounters];
 #pragma unroll
   for (int k = 0; k < kCounters; k++) sum[k] = 0;
-  for (uint32_t x = b0; x < b1; x++)
+  uint32_t mask = 0;
+  for (uint32_t x = b0; x < b1; x++) {
 #pragma unroll
-    for (int k = 0; k < kCounters; k++) sum[k] += b.blk_counts[(size_t)x * kCounters + k];
+    for (int k = 0; k < kCounters; k++) sum[k] += b.blk_counts[(size_t)x * kTileWords + k];
+    mask = join_masks(mask, b.blk_counts[(size_t)x * kTileWords + kCounters]);
+  }
+  uint32_t minc = mask;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, minc, o);
+    if (lane >= o) minc = join_masks(t, minc);
+  }
+  uint32_t mexcl = __shfl_up_sync(0xffffffffu, minc, 1);
+  if (lane == 0) mexcl = 0u;
+  if (lane == 31) s_mask[warp] = minc;
   uint32_t excl[kCounters];
 #pragma unroll
   for (int k = 0; k < kCounters; k++) {
@@ -178,13 +227,19 @@ __global__ void __launch_bounds__(kScanThreads)
   __syncthreads();
 #pragma unroll
   for (int k = 0; k < kCounters; k++) excl[k] += s_warp[warp][k];
-  for (uint32_t x = b0; x < b1; x++)
+  uint32_t mpre = 0;
+  for (int w = 0; w < warp; w++) mpre = join_masks(mpre, s_mask[w]);
+  mask = join_masks(mpre, mexcl);
+  for (uint32_t x = b0; x < b1; x++) {
 #pragma unroll
     for (int k = 0; k < kCounters; k++) {
-      const uint32_t c = b.blk_counts[(size_t)x * kCounters + k];
-      b.blk_offs[(size_t)x * kCounters + k] = excl[k];
+      const uint32_t c = b.blk_counts[(size_t)x * kTileWords + k];
+      b.blk_offs[(size_t)x * kTileWords + k] = excl[k];
       excl[k] += c;
     }
+    b.blk_offs[(size_t)x * kTileWords + kCounters] = mask >> 16;
+    mask = join_masks(mask, b.blk_counts[(size_t)x * kTileWords + kCounters]);
+  }
   if (tid == 0) {
     TreeMeta m;
     uint32_t run = 0, levels = 0;
@@ -206,7 +261,7 @@ __global__ void __launch_bounds__(kScanThreads)
   }
 }
 
-// K3: node indices, parents, child bases, leaf lists.
+// K3 of the stateless builds: node indices, parents, child bases, leaf lists.
 __global__ void __launch_bounds__(kFlagThreads) tree_emit_kernel(BuildBuffers b, Layout Lo,
                                                                   DevState* st) {
   griddep_wait();  // launched with a programmatic dependency: predecessors' writes first
@@ -248,7 +303,7 @@ __global__ void __launch_bounds__(kFlagThreads) tree_emit_kernel(BuildBuffers b,
   }
   __syncthreads();
   if (tid < kCounters) {
-    uint32_t run = b.blk_offs[(size_t)tile * kCounters + tid];
+    uint32_t run = b.blk_offs[(size_t)tile * kTileWords + tid];
     for (int w = 0; w < kFlagThreads / 32; w++) {
       const uint32_t t = s_warp[w][tid];
       s_warp[w][tid] = run;
@@ -338,7 +393,7 @@ __device__ __forceinline__ WalkInfo walk_info(float size, uint32_t child, uint32
   return w;
 }
 
-// K4: one thread per leaf slot (a block per build tile, kLeafThreads = one
+// K4 of the stateless builds and of gs_refresh: one thread per leaf slot (a block per build tile, kLeafThreads = one
 // tile); leaf COM, then carry each finished node to its parent; the last child
 // to finish sums the parent (children in slot order).
 constexpr int kLeafThreads = kFlagTile;

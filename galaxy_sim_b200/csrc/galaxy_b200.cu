@@ -33,6 +33,7 @@
 #include "morton.cuh"
 #include "particles.cuh"
 #include "sort.cuh"
+#include "tile_tree.cuh"
 #include "walk.cuh"
 
 using namespace gs;
@@ -107,7 +108,7 @@ uint64_t plan_bytes(const Plan& p) {
   b += c * (2 * 32 + 2 * 16 + 4 + 16 + 4 + 4);   // particles x2, stellar x2, energy, compact, perm, inv
   b += c * (4 * 4 + 1 + 2 * 4) + 2 * 4 + 4;     // keys x2, vals x2, dl, leaf lists
   b += p.sort_words * 4;
-  b += (uint64_t)p.flag_tiles * (6 * 4 + 2 * kCounters * 4);
+  b += (uint64_t)p.flag_tiles * (6 * 4 + 2 * kTileWords * 4);
   b += n * (16 + 16 + 4 + 4 + 4 + 1 + 4) + 4;   // cm, info, node_start, child_base, parent, depth, arrive
   b += s * (sizeof(DevState) + sizeof(TreeMeta) + sizeof(MortonFrame) + 4 + kPartials * 8 + sizeof(SegDesc));
   b += (uint64_t)(p.sort_tiles + p.flag_tiles + p.groups) * 4;
@@ -466,8 +467,8 @@ int pool_init(gs_ctx* c, int device, uint64_t cap, uint32_t slots) {
   A(c->bbox_part, (size_t)p.flag_tiles * 6);
   A(c->frames, p.slots);
   A(c->dl, p.cap + 4);
-  A(c->blk_counts, (size_t)p.flag_tiles * kCounters);
-  A(c->blk_offs, (size_t)p.flag_tiles * kCounters);
+  A(c->blk_counts, (size_t)p.flag_tiles * kTileWords);
+  A(c->blk_offs, (size_t)p.flag_tiles * kTileWords);
   A(c->node_start, p.nodes);
   A(c->child_base, p.nodes + 1);
   A(c->parent, p.nodes);
@@ -705,22 +706,16 @@ void enqueue_sort_passes(gs_ctx* c, bool inv, uint32_t spin_limit = kSpinLimit, 
   else sort_passes_items<16>(c, inv, spin_limit, withhold);
 }
 
-// the trees over keys[0] (sorted codes) with COM from pos; root size from the
-// Morton frames of the preceding sort (frames) or root_size.
-void enqueue_build(gs_ctx* c, const float4* pos, uint32_t stride, int com_mode, double root_size,
-                   const MortonFrame* frames) {
+// the trees of the stateless builds over keys[0] (sorted codes), with MortonTree.build's
+// COM from pos; root size from the Morton frames of the preceding sort (frames) or root_size.
+void enqueue_build(gs_ctx* c, const float4* pos, uint32_t stride, double root_size, const MortonFrame* frames) {
   const Layout& L = c->lay;
   cudaStream_t s = c->stream;
   BuildBuffers b = c->bb();
   launch_pdl(tree_flags_kernel, L.flag_tiles, kFlagThreads, s, b, L);
   launch_pdl(tree_scan_kernel, L.nseg, kScanThreads, s, b, L, root_size, frames, c->st);
   launch_pdl(tree_emit_kernel, L.flag_tiles, kFlagThreads, s, b, L, c->st);
-  if (com_mode == kComJs)
-    launch_pdl(tree_leaves_kernel<kComJs>, L.flag_tiles, kLeafThreads, s, b, L, pos, stride, c->st);
-  else if (com_mode == kComF64)
-    launch_pdl(tree_leaves_kernel<kComF64>, L.flag_tiles, kLeafThreads, s, b, L, pos, stride, c->st);
-  else
-    launch_pdl(tree_leaves_kernel<kComF32>, L.flag_tiles, kLeafThreads, s, b, L, pos, stride, c->st);
+  launch_pdl(tree_leaves_kernel<kComJs>, L.flag_tiles, kLeafThreads, s, b, L, pos, stride, c->st);
 }
 
 template <int LPP>
@@ -824,15 +819,22 @@ void enqueue_sort_build(gs_ctx* c, int advance_time) {
   }
   enqueue_codes_sort(c, c->part[c->cur], 2, advance_time);
   enqueue_sort_passes(c, track);
-  launch_pdl(gather_kernel, L.flag_tiles, kTileThreads, c->stream, (const uint32_t*)c->vals[0],
+  const BuildBuffers bb = c->bb();
+  launch_pdl(gather_flags_kernel, L.flag_tiles, kTileThreads, c->stream, (const uint32_t*)c->vals[0],
              (const float4*)c->part[c->cur], c->part[c->cur ^ 1], (const float4*)c->stel[c->scur],
-             c->stel[c->scur ^ 1], L, c->st);
+             c->stel[c->scur ^ 1], L, c->st, bb);
   c->cur ^= 1;
   c->scur ^= 1;
   if (track)
     launch_pdl(track_kernel, cdiv(L.nseg, 128), 128, c->stream, (const uint32_t*)c->inv,
                (const float4*)c->part[c->cur], L, c->st);
-  enqueue_build(c, c->part[c->cur], 2, c->com_mode, 0.0, c->frames);
+  launch_pdl(tree_scan_kernel, L.nseg, kScanThreads, c->stream, bb, L, 0.0, (const MortonFrame*)c->frames, c->st);
+  if (c->com_mode == kComF64)
+    launch_pdl(tree_tile_kernel<kComF64>, L.flag_tiles, kFlagThreads, c->stream, bb, L,
+               (const float4*)c->part[c->cur], c->st);
+  else
+    launch_pdl(tree_tile_kernel<kComF32>, L.flag_tiles, kFlagThreads, c->stream, bb, L,
+               (const float4*)c->part[c->cur], c->st);
 }
 
 // Params upload: sim_time follows Params.time and tracked halo centres keep their
@@ -2066,7 +2068,7 @@ int gs_tree_build(const uint32_t* sorted_codes, const float* pos3, const float* 
   }
   TK(cudaMemcpyAsync(c->part[0], h.data(), sizeof(float4) * N, cudaMemcpyHostToDevice, c->stream), "upload");
   TK(cudaMemcpyAsync(c->keys[0], k.data(), sizeof(uint32_t) * N, cudaMemcpyHostToDevice, c->stream), "codes");
-  enqueue_build(c, c->part[0], 1, kComJs, root_size, nullptr);
+  enqueue_build(c, c->part[0], 1, root_size, nullptr);
   TK(cudaGetLastError(), "build");
   return tree_outputs(t, max_nodes, nodes, num_nodes, level_ranges, lr_cap, n_levels);
 }
@@ -2097,7 +2099,7 @@ int gs_sort_and_build(const float* particles8, const float* stellar4, uint32_t N
   enqueue_codes_sort(c, P, 2, 0);
   enqueue_sort_passes(c, false);
   gather_kernel<<<c->lay.flag_tiles, kTileThreads, 0, c->stream>>>(c->vals[0], P, P2, S, S2, c->lay, c->st);
-  enqueue_build(c, P2, 2, kComJs, 0.0, c->frames);
+  enqueue_build(c, P2, 2, 0.0, c->frames);
   TK(cudaGetLastError(), "sort and build");
   std::vector<uint32_t> hp(perm ? 0 : N);
   uint32_t* const pm = perm ? perm : hp.data();

@@ -203,11 +203,9 @@ __global__ void __launch_bounds__(kTileThreads)
 // Gather dst[i] = src[perm[i]] of the 32-byte particle and 16-byte stellar
 // records (nbody_bh.wgsl:322-326, :336-340). perm holds pool indices of the
 // same galaxy; anything else is flagged, never dereferenced.
-__global__ void __launch_bounds__(kTileThreads)
-    gather_kernel(const uint32_t* __restrict__ perm, const float4* __restrict__ pin,
-                  float4* __restrict__ pout, const float4* __restrict__ sin,
-                  float4* __restrict__ sout, Layout L, DevState* st) {
-  griddep_wait();  // launched with a programmatic dependency: predecessors' writes first
+__device__ __forceinline__ void tile_gather(const uint32_t* __restrict__ perm, const float4* __restrict__ pin,
+                                            float4* __restrict__ pout, const float4* __restrict__ sin,
+                                            float4* __restrict__ sout, const Layout& L, DevState* st) {
   const TileRange t = tile_range(L, blockIdx.x);
 #pragma unroll
   for (int q = 0; q < kTilePer; q++) {
@@ -223,6 +221,23 @@ __global__ void __launch_bounds__(kTileThreads)
     pout[2 * (size_t)i + 1] = b;
     if (sout) sout[i] = sin[s];
   }
+}
+__global__ void __launch_bounds__(kTileThreads)
+    gather_kernel(const uint32_t* __restrict__ perm, const float4* __restrict__ pin,
+                  float4* __restrict__ pout, const float4* __restrict__ sin,
+                  float4* __restrict__ sout, Layout L, DevState* st) {
+  griddep_wait();  // launched with a programmatic dependency: predecessors' writes first
+  tile_gather(perm, pin, pout, sin, sout, L, st);
+}
+
+// The gather with the tree's tile flags: both follow the sort and neither needs the other.
+__global__ void __launch_bounds__(kTileThreads)
+    gather_flags_kernel(const uint32_t* __restrict__ perm, const float4* __restrict__ pin,
+                        float4* __restrict__ pout, const float4* __restrict__ sin,
+                        float4* __restrict__ sout, Layout L, DevState* st, BuildBuffers b) {
+  griddep_wait();  // launched with a programmatic dependency: predecessors' writes first
+  tile_gather(perm, pin, pout, sin, sout, L, st);
+  tile_flags(b, L);
 }
 
 // Central-particle tracking after a sort (one thread per galaxy): the tracked
