@@ -186,7 +186,7 @@ struct WalkSmem {
       // words: cxy[4p..4p+3] = {x(2p), x(2p+1), y(2p), y(2p+1)}, czm likewise {z, m}
       __align__(16) float cxy[16 * kWalkRanges];
       __align__(16) float czm[16 * kWalkRanges];
-      float cs2[8 * kWalkRanges];
+      float cthr[8 * kWalkRanges];  // accepted where r^2 + eps^2 (groups of 32) or theta^2 times it is larger
     };
     uint2 pinfo[kLeafWindow];       // a window's source pairs: {first source | both << 31, opening mask}
   };
@@ -419,6 +419,25 @@ __device__ inline uint32_t set_gt_mask(float a, float b) {
   return r;
 }
 
+// The largest finite x >= 0 for which theta2 * x > s2 does not hold in FP32 (the product
+// grows with x): x > open_threshold(s2, theta2) decides like theta2 * x > s2 for every x
+// but infinity with theta2 = 0. Searched on the bits, from around s2 / theta2.
+__device__ __noinline__ float open_threshold(float s2, float theta2) {
+  uint32_t lo = 0u, hi = 0x7f7fffffu;  // holds not at lo
+  if (!(theta2 * __uint_as_float(hi) > s2)) return __uint_as_float(hi);
+  const uint32_t q = __float_as_uint(s2 / theta2);
+  if (q - 8u < 0x7f000000u) {
+    if (!(theta2 * __uint_as_float(q - 4u) > s2)) lo = q - 4u;
+    if (theta2 * __uint_as_float(q + 4u) > s2) hi = q + 4u;
+  }
+  while (hi - lo > 1u) {
+    const uint32_t mid = lo + (hi - lo) / 2u;
+    if (theta2 * __uint_as_float(mid) > s2) hi = mid;
+    else lo = mid;
+  }
+  return __uint_as_float(lo);
+}
+
 // Transpose of the 32 x 32 bit matrix held one row per lane: afterwards bit j
 // of lane i is bit i of lane j (five butterfly stages of 16, 8, 4, 2, 1 bits). The
 // stages of 16 and 8 bits are one byte permutation each, the others a rotation and a
@@ -470,6 +489,30 @@ __global__ void __launch_bounds__(kWalkThreads, COMP ? kWalkResident - 1 : kWalk
   const unsigned full = 0xffffffffu;
 
   const uint32_t below = (1u << lane) - 1u, lanebit = 1u << pl;
+  // Walk groups of 32 test size^2 < theta^2 (r^2 + eps^2) as r^2 + eps^2 > thr(size^2), with the
+  // threshold (open_threshold) that makes every decision the same. A tree's sizes are the
+  // root's over powers of two, so its size^2 share a mantissa, and the threshold's bits
+  // are size^2's plus one number for all of them; other sizes (uploaded trees) are
+  // searched for. It saves a packed multiply per pair; a warp of smaller groups walks too
+  // few pairs to earn back the set-up (walk of 524288 particles 972 -> 951 us; of 60001, in
+  // groups of 16, 99 -> 101) and multiplies by theta^2, kept above zero so that an inactive lane's
+  // infinite distance is always far.
+  constexpr bool kThr = LPP == 1;
+  float theta2;
+  uint32_t root_s2 = 0, thr_add = 0, thr_range = 0, thr_slot = 0xffffffffu;
+  auto threshold_of = [&](const SegDesc& g) {
+    const float theta = __ldg(&a.st[g.slot].p.theta);
+    theta2 = theta * theta;
+    if (!kThr) {
+      theta2 = fmaxf(theta2, 1.17549435e-38f);
+      return;
+    }
+    root_s2 = __float_as_uint(a.info[g.node_off].s2);
+    thr_add = __float_as_uint(open_threshold(__uint_as_float(root_s2), theta2)) - root_s2;
+    // both ends far from subnormals and infinity: size^2 within [2^-95, 2^93), the shift within 2^+-16
+    thr_range = root_s2 - 0x10000000u < 0x5e000000u && thr_add + 0x08000000u < 0x10000000u ? 0x5e000000u : 0u;
+  };
+  if (ONE) threshold_of(a.seg0);
   if (lane < kWalkRanges) S.stack[lane] = make_uint2(0u, 0u);
 
   while (true) {
@@ -484,7 +527,6 @@ __global__ void __launch_bounds__(kWalkThreads, COMP ? kWalkResident - 1 : kWalk
     DevState* const sst = a.st + sd.slot;
     const gs_params& P = sst->p;  // read-only during the walk; fields loaded where used
     const float eps2p = __ldg(&P.epsilon2);
-    const float theta2 = __ldg(&P.theta) * __ldg(&P.theta);
     const float qe2 = 0.25f * eps2p;
     // Self pairs may be summed and removed afterwards when softened. Softening below
     // the smallest normal float counts as none, so every r^2 + eps^2 below is a
@@ -496,6 +538,10 @@ __global__ void __launch_bounds__(kWalkThreads, COMP ? kWalkResident - 1 : kWalk
     // normal float instead, which moves no r^2 above 1e-30 by more than a
     // rounding step, and such a node is opened as before.
     const float eps2 = soft ? eps2p : 1.17549435e-38f;
+    if (!ONE && sd.slot != thr_slot) {  // a warp's next item is mostly of the same galaxy
+      threshold_of(sd);
+      thr_slot = sd.slot;
+    }
     const uint32_t seg_end = sd.off + sd.n;
     const uint32_t gbeg = sd.off + (gcur - sd.group0) * kWalkGroup + part * G, gend = gbeg + G;
     const uint32_t i = gbeg + pl;
@@ -559,7 +605,7 @@ __global__ void __launch_bounds__(kWalkThreads, COMP ? kWalkResident - 1 : kWalk
       // Stage range r in lanes 8r..8r+7: one child per lane; slots past a range's
       // count hold massless dummies. Massless and sub-softening children
       // (size^2 < eps^2/4, always accepted, nbody_bh.wgsl:112) get size^2 = -inf,
-      // so the per-lane test is the single compare size^2 < theta^2 (r^2 + eps^2).
+      // so the per-lane test is one compare with the child's threshold.
       bool own = false, isleaf = false, massive = false, skip = false;
       uint32_t cnode = 0, cchild = 0, ccnt = 0;  // this lane's slot: node, first child or particle, count
       float csize = 1.f;
@@ -567,63 +613,51 @@ __global__ void __launch_bounds__(kWalkThreads, COMP ? kWalkResident - 1 : kWalk
         const uint32_t c = lane & 7;
         const uint2 e = top[-(lane >> 3)];
         const uint32_t rs = e.x & 0x1fffffffu;
-        float4 q = make_float4(1e30f, 1e30f, 1e30f, 0.f);
-        WalkInfo w;
-        w.s2 = 0.f;
-        w.child = 0;
-        w.info = kLeafBit;
-        w.size = 1.f;
+        // slots past the count (and empty entries) load a node of the range (the first of
+        // the pool) and are made dummies like massless nodes
         bool real = e.y != 0u && c <= e.x >> 29, counted = true;
+        cnode = rs + min(c, e.x >> 29);
         if (NS > 1 && real) {
-          const uint32_t node = rs + c;
-          if (node < up_end) counted = ksp == 0;                                    // levels above the split
-          else if (node < win_end && ((node - up_end) & (NS - 1)) != ksp) real = false;  // another split's
+          if (cnode < up_end) counted = ksp == 0;                                    // levels above the split
+          else if (cnode < win_end && ((cnode - up_end) & (NS - 1)) != ksp) real = false;  // another split's
         }
-        if (real) {
-          q = __ldg(&a.cm[rs + c]);
-          w = a.info[rs + c];
-        }
-        cnode = rs + c;
-        cchild = w.child;
-        ccnt = w.info & ~kLeafBit;
-        csize = w.size;
-        isleaf = real && (w.info & kLeafBit);
-        massive = real && q.w != 0.0f && counted;
+        float4 q = __ldg(&a.cm[cnode]);
+        const uint4 w = __ldg(reinterpret_cast<const uint4*>(a.info) + cnode);  // WalkInfo
+        cchild = w.y;
+        ccnt = w.z & ~kLeafBit;
+        csize = __uint_as_float(w.w);
+        const bool heavy = real && q.w != 0.0f;
+        isleaf = real && (w.z & kLeafBit);
+        massive = heavy && counted;
         skip = isleaf && !counted;
-        own = isleaf && q.w != 0.0f && cchild < gend && cchild + ccnt > gbeg;
-        float s2 = w.s2;
-        if (q.w == 0.0f) {  // never opened, contributes nothing (far away, massless)
-          s2 = -INFINITY;
-          q = make_float4(1e30f, 1e30f, 1e30f, 0.f);
-        } else if (s2 < qe2) {
-          s2 = -INFINITY;
+        own = isleaf && heavy && cchild < gend && cchild + ccnt > gbeg;
+        const float s2 = __uint_as_float(w.x);
+        // never opened: massless and dummies (which contribute nothing, far away and
+        // massless), and sub-softening children
+        float thr = -INFINITY;
+        if (heavy && !(s2 < qe2)) {
+          thr = kThr ? __uint_as_float(w.x + thr_add) : s2;
+          if (kThr && (((w.x ^ root_s2) & 0x7fffffu) || w.x - 0x10000000u >= thr_range)) thr = open_threshold(s2, theta2);
         }
+        if (!heavy) q = make_float4(1e30f, 1e30f, 1e30f, 0.f);
         const int st = 4 * (lane >> 1) + (lane & 1);
         S.cxy[st] = q.x;
         S.cxy[st + 2] = q.y;
         S.czm[st] = q.z;
         S.czm[st + 2] = counted ? q.w : 0.0f;  // tested for opening, adds nothing
-        S.cs2[lane] = s2;
+        S.cthr[lane] = thr;
       }
       const unsigned ownmask = __ballot_sync(full, own);  // leaves holding our particles
       const unsigned leafmask = __ballot_sync(full, isleaf);
       const unsigned massmask = DBG ? __ballot_sync(full, massive) : 0u;
       const unsigned skipm = NS > 1 ? __ballot_sync(full, skip) : 0u;  // opened leaves another split sums
       __syncwarp();
-      // per range: this lane active; the slots whose open bits this lane keeps (its
-      // active ranges' eight slots: a slot past a range's count holds a dummy of
-      // size^2 -inf, which every active lane accepts, so it never sets an open bit)
-      // theta^2 per range; a lane inactive for a range tests against -inf, so its
-      // td is -inf (or NaN) and it accepts and adds nothing there
-      uint32_t act = 0;
-      float th2[kWalkRanges];
+      // eps^2 per range; a lane inactive for a range adds +inf: it accepts every child, and
+      // adds nothing as rsqrt gives 0, and so it sets no open bit (nor does a slot past a
+      // range's count, a dummy with the threshold -inf)
+      float e2[kWalkRanges];
 #pragma unroll
-      for (int r = 0; r < kWalkRanges; r++) {
-        const bool on = masks[r] & lanebit;
-        th2[r] = on ? theta2 : -INFINITY;
-        if (on) act |= 0xffu << (8 * r);
-      }
-      const uint32_t keep = act & mine;
+      for (int r = 0; r < kWalkRanges; r++) e2[r] = masks[r] & lanebit ? eps2 : INFINITY;
       uint32_t obits = 0;  // children this lane opens (active, not accepted), bit = slot
       // COMP: the round's far-field terms (at most 32 per lane) are summed plainly,
       // then the round's sum joins the particle's total in one Kahan step
@@ -635,18 +669,18 @@ __global__ void __launch_bounds__(kWalkThreads, COMP ? kWalkResident - 1 : kWalk
         const int pp = (int)sub + kk * LPP;
         const int c = 2 * pp;
         // the pair's range pp >> 2: (kk * LPP) >> 2 for shares below 4, one more above
-        const float t2 = LPP < 8 ? th2[(kk * LPP) >> 2] : (sub >= 4 ? th2[2 * kk + 1] : th2[2 * kk]);
+        const float er = LPP < 8 ? e2[(kk * LPP) >> 2] : (sub >= 4 ? e2[2 * kk + 1] : e2[2 * kk]);
         const float4 qxy = *reinterpret_cast<const float4*>(&S.cxy[2 * c]);
         const float4 qzm = *reinterpret_cast<const float4*>(&S.czm[2 * c]);
         const float2 qx = make_float2(qxy.x, qxy.y), qy = make_float2(qxy.z, qxy.w);
         const float2 qz = make_float2(qzm.x, qzm.y), qm = make_float2(qzm.z, qzm.w);
-        const float2 s2 = *reinterpret_cast<const float2*>(&S.cs2[c]);
+        const float2 thr = *reinterpret_cast<const float2*>(&S.cthr[c]);
         const float2 rx = __fadd2_rn(qx, px), ry = __fadd2_rn(qy, py), rz = __fadd2_rn(qz, pz);
-        const float2 d2 = __ffma2_rn(rx, rx, __ffma2_rn(ry, ry, __ffma2_rn(rz, rz, f2(eps2))));
-        const float2 td = __fmul2_rn(f2(t2), d2);
+        const float2 d2 = __ffma2_rn(rx, rx, __ffma2_rn(ry, ry, __ffma2_rn(rz, rz, f2(er))));
         // all ones where the child is accepted; an accepted child keeps r^2 + eps^2,
         // any other gets +inf, so rsqrt makes its terms exactly 0
-        const uint32_t ax_ = set_gt_mask(td.x, s2.x), ay_ = set_gt_mask(td.y, s2.y);
+        const float2 td = kThr ? d2 : __fmul2_rn(f2(theta2), d2);
+        const uint32_t ax_ = set_gt_mask(td.x, thr.x), ay_ = set_gt_mask(td.y, thr.y);
         obits |= (~ax_ & (1u << c)) | (~ay_ & (2u << c));
         const float2 dsel = make_float2(__uint_as_float((__float_as_uint(d2.x) & ax_) | (0x7f800000u & ~ax_)),
                                         __uint_as_float((__float_as_uint(d2.y) & ay_) | (0x7f800000u & ~ay_)));
@@ -671,9 +705,13 @@ __global__ void __launch_bounds__(kWalkThreads, COMP ? kWalkResident - 1 : kWalk
         kahan_add2(F.az, caz, raz);
         kahan_add2(F.pt, cpt, rpt);
       }
-      obits &= keep;
       const uint32_t om = __reduce_or_sync(full, obits);  // children opened by some lane
-      if (DBG) {  // keep holds this lane's slots only
+      if (DBG) {
+        uint32_t keep = 0;  // the slots this lane tests, of the ranges it is active for
+#pragma unroll
+        for (int r = 0; r < kWalkRanges; r++)
+          if (masks[r] & lanebit) keep |= 0xffu << (8 * r);
+        keep &= mine;
         nvisit += __popc(massmask & keep);
         nmono += __popc(massmask & keep & ~obits);
       }
@@ -681,7 +719,7 @@ __global__ void __launch_bounds__(kWalkThreads, COMP ? kWalkResident - 1 : kWalk
         const uint32_t cc = __ffs(bb) - 1;
         const uint32_t lf = __shfl_sync(full, cchild, cc), cnt = __shfl_sync(full, ccnt, cc);
         const float sz = __shfl_sync(full, csize, cc);
-        if (((act >> cc) & 1u) && (i - lf) < cnt) {
+        if ((top[-(int)(cc >> 3)].y & lanebit) && (i - lf) < cnt) {
           dens = (float)cnt / (sz * sz * sz);
           // the leaf's direct sum includes the particle itself (softened walks)
           if (((obits & ~skipm) >> cc) & 1u) selfw += 1.0f;
