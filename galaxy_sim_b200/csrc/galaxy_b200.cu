@@ -1381,8 +1381,8 @@ int gs_star_formation(gs_ctx* ctx) {
   int rc = ensure_layout(ctx);
   if (rc) return rc;
   if (!ctx->lay.nseg) return GS_OK;
-  sf_kernel<<<ctx->lay.flag_tiles, kTileThreads, 0, ctx->stream>>>(ctx->part[ctx->cur], ctx->stel[ctx->scur],
-                                                                    ctx->lay, ctx->st);
+  launch_pdl(sf_kernel, ctx->lay.flag_tiles, kTileThreads, ctx->stream, ctx->part[ctx->cur], ctx->stel[ctx->scur],
+             ctx->lay, (const DevState*)ctx->st);
   CK(ctx, cudaGetLastError(), "star formation");
   return GS_OK;
 }
@@ -1393,8 +1393,9 @@ int gs_read_positions(gs_ctx* ctx, float* out4, uint64_t timeout_ns) {
   if (!out4) return ctx->fail(GS_EINVAL, "out4 is NULL");
   // an asynchronous readback still copying out of the compaction buffer finishes first
   if (ctx->rb_pending) CK(ctx, cudaStreamWaitEvent(ctx->stream, ctx->rb_done, 0), "readback order");
-  compact_kernel<<<grid_for(s->n, 256, 148 * 16), 256, 0, ctx->stream>>>(
-      ctx->part[ctx->cur] + 2 * (size_t)s->off, ctx->energy + s->off, ctx->compact + s->off, s->n);
+  launch_pdl(compact_kernel, grid_for(s->n, 256, 148 * 16), 256, ctx->stream,
+             (const float4*)ctx->part[ctx->cur] + 2 * (size_t)s->off, (const float*)ctx->energy + s->off,
+             ctx->compact + s->off, s->n, (const double*)nullptr, (const unsigned*)nullptr, (double*)nullptr);
   CK(ctx, cudaGetLastError(), "compact");
   int rc = wait_stream(ctx, timeout_ns, s);
   if (rc) return rc;
@@ -1421,12 +1422,11 @@ int gs_encode_position_readback(gs_ctx* ctx, float* out4, gs_diag* diag) {
   }
   // in stream order: vec4(pos, e_i) into the compaction buffer and the diagnostics
   // snapshot; the copy stream then moves the positions while later steps run
-  compact_kernel<<<grid_for(s->n, 256, 148 * 16), 256, 0, ctx->stream>>>(
-      ctx->part[ctx->cur] + 2 * (size_t)s->off, ctx->energy + s->off, ctx->compact + s->off, s->n);
+  launch_pdl(compact_kernel, grid_for(s->n, 256, 148 * 16), 256, ctx->stream,
+             (const float4*)ctx->part[ctx->cur] + 2 * (size_t)s->off, (const float*)ctx->energy + s->off,
+             ctx->compact + s->off, s->n, (const double*)ctx->diag_out + (size_t)ctx->sel * kPartials,
+             (const unsigned*)&ctx->st[ctx->sel].err, ctx->rb_host_dev);
   CK(ctx, cudaGetLastError(), "compact");
-  readback_snapshot_kernel<<<1, 32, 0, ctx->stream>>>(ctx->diag_out + (size_t)ctx->sel * kPartials,
-                                                      &ctx->st[ctx->sel].err, ctx->rb_host_dev);
-  CK(ctx, cudaGetLastError(), "readback snapshot");
   CK(ctx, cudaEventRecord(ctx->rb_ready, ctx->stream), "readback event");
   CK(ctx, cudaStreamWaitEvent(ctx->rb_stream, ctx->rb_ready, 0), "readback order");
   CK(ctx, cudaMemcpyAsync(out4, ctx->compact + s->off, (size_t)s->n * 16, cudaMemcpyDeviceToHost, ctx->rb_stream),

@@ -279,6 +279,7 @@ __global__ void track_kernel(const uint32_t* __restrict__ inv, const float4* __r
 __global__ void __launch_bounds__(kTileThreads)
     sf_kernel(float4* __restrict__ P, float4* __restrict__ S, Layout L,
               const DevState* __restrict__ st) {
+  griddep_wait();  // launched with a programmatic dependency: predecessors' writes first
   const TileRange t = tile_range(L, blockIdx.x);
   if (st[t.slot].sf_off) return;
   const gs_params prm = st[t.slot].p;
@@ -295,23 +296,23 @@ __global__ void __launch_bounds__(kTileThreads)
   }
 }
 
-// compact_positions (nbody_bh.wgsl:188-195) over one particle range.
-__global__ void compact_kernel(const float4* __restrict__ P, const float* __restrict__ energy,
-                               float4* __restrict__ out, uint32_t N) {
+// compact_positions (nbody_bh.wgsl:188-195) over one particle range. With `host`, also a
+// snapshot of the galaxy's diagnostics (kPartials doubles) and error word into mapped
+// pinned host memory, in stream order: the asynchronous readback delivers the values of
+// the step it follows even when later steps overwrite them.
+__global__ void __launch_bounds__(256)
+    compact_kernel(const float4* __restrict__ P, const float* __restrict__ energy, float4* __restrict__ out, uint32_t N,
+                   const double* __restrict__ diag, const unsigned* __restrict__ err, double* host) {
+  griddep_wait();  // launched with a programmatic dependency: predecessors' writes first
+  if (host && blockIdx.x == 0) {
+    const int t = threadIdx.x;
+    if (t < kPartials) host[t] = diag[t];
+    if (t == kPartials) reinterpret_cast<unsigned*>(host + kPartials)[0] = *err;
+  }
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
     const float4 p = P[2 * (size_t)i];
     out[i] = make_float4(p.x, p.y, p.z, energy[i]);
   }
-}
-
-// Snapshot of one galaxy's diagnostics (kPartials doubles) and error word into
-// mapped pinned host memory, in stream order: the asynchronous readback delivers
-// the values of the step it follows even when later steps overwrite them.
-__global__ void readback_snapshot_kernel(const double* __restrict__ diag, const unsigned* __restrict__ err,
-                                         double* host) {
-  const int t = threadIdx.x;
-  if (t < kPartials) host[t] = diag[t];
-  if (t == kPartials) reinterpret_cast<unsigned*>(host + kPartials)[0] = *err;
 }
 
 // refresh_level (nbody_bh.wgsl:288-313) on one BFS level of the walk layout
