@@ -57,13 +57,20 @@ constexpr int kWalkRanges = GS_WALK_RANGES;  // child ranges popped and tested p
 static_assert(kWalkRanges >= 1 && kWalkRanges <= 4, "a round stages at most one child per lane");
 // ranges; a round explores kWalkRanges paths, each leaving <= 7 pending ranges per depth
 constexpr int kWalkStack = 8 * 11 * kWalkRanges;
-// Resident blocks per SM the walk is compiled for: 72 registers per thread without
-// spills, and 31.5 KB of staging per block, of which 7 fit an SM. The launch tuning
-// accepts 1..8; more than the resident blocks launch no further ones. (Before leaf
-// sums were queued, a second build of 64 registers for 8 blocks ran the 96-galaxy
-// pool in 7.569 ms against 7.572 ms for this one.)
+// Resident blocks per SM the walk is compiled for. Walk groups of 32: 7, the most that 31.7
+// KB of staging per block let onto an SM, at 72 registers per thread (6 at 80 registers:
+// walk of 524288 particles 953 -> 968 us; compensated sums need the 80: 306 -> 290 us on a
+// sphere of 200003). Smaller groups walk small galaxies, which do not fill the SMs, and
+// run without spills and with more loads in flight at more registers: full step at 7 / 6
+// / 5 blocks in us: 4096 particles 62.1 / 61.2 / 60.0, 16384 106.0 / 101.1 / 101.8, 25000 133 / 131 / 124
+// (groups of 8); 60001 163 / 157 / 164, 100000 310 / 308 / 303 (groups of 16). The launch
+// tuning accepts 1..8 blocks per SM; more than the resident ones launch no further ones.
 constexpr int kWalkBlocksPerSM = 8;
-constexpr int kWalkResident = 7;  // 6 with compensated sums (80 registers: 306 -> 290 us on a sphere of 200003)
+constexpr int kWalkResident = 7;
+template <int LPP, bool COMP>
+constexpr int walk_resident() {
+  return LPP >= 4 ? 5 : LPP == 2 || COMP ? 6 : kWalkResident;
+}
 constexpr uint32_t kWalkGroup = 32;             // particles per walk group (layout, diagnostics)
 constexpr uint32_t kWalkParts = 8;              // partial-sum slots per walk group (the largest LPP)
 // with the walk group chosen by size, galaxies of at most this many particles
@@ -342,6 +349,7 @@ __device__ __forceinline__ void leaf_flush(Smem& S, const float4* __restrict__ p
         }
         if (lane < (int)SH) S.list[n + lane] = 0u;
       }
+      if (NSUB > 1 && n == 0) continue;  // no pair of this subgroup's
       __syncwarp();
       const float2 px = f2(NSUB > 1 ? __shfl_sync(full, nx, SUBT * g + tl) : nx);
       const float2 py = f2(NSUB > 1 ? __shfl_sync(full, ny, SUBT * g + tl) : ny);
@@ -465,7 +473,7 @@ __device__ __forceinline__ uint32_t warp_transpose(uint32_t x, int lane) {
 // LPP: lanes per particle (walk group of 32 / LPP particles); a launch walks the
 // galaxies whose SegDesc wlpp field equals LPP and skips the others' work items.
 template <bool SF, bool DBG, bool ONE, bool COMP, int LPP>
-__global__ void __launch_bounds__(kWalkThreads, COMP ? kWalkResident - 1 : kWalkResident) walk_kernel(WalkArgs a) {
+__global__ void __launch_bounds__(kWalkThreads, walk_resident<LPP, COMP>()) walk_kernel(WalkArgs a) {
   static_assert(LPP == 1 || LPP == 2 || LPP == 4 || LPP == 8, "lanes per particle");
   constexpr uint32_t G = 32 / LPP;                         // particles per work item
   constexpr int NPP = 16 / LPP;                            // slot pairs a lane tests in a full round
