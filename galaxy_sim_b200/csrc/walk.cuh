@@ -616,13 +616,15 @@ __global__ void __launch_bounds__(kWalkThreads, walk_resident<LPP, COMP>()) walk
       // so the per-lane test is one compare with the child's threshold.
       bool own = false, isleaf = false, massive = false, skip = false;
       uint32_t cnode = 0, cchild = 0, ccnt = 0;  // this lane's slot: node, first child or particle, count
+      uint32_t act = 0;                          // and the particles that opened its parent
       float csize = 1.f;
       if (lane < 8 * kWalkRanges) {
         const uint32_t c = lane & 7;
         const uint2 e = top[-(lane >> 3)];
         const uint32_t rs = e.x & 0x1fffffffu;
+        act = e.y;
         // slots past the count (and empty entries) load a node of the range (the first of
-        // the pool) and are made dummies like massless nodes
+        // the pool) and are made dummies like massless nodes, with no children to go on to
         bool real = e.y != 0u && c <= e.x >> 29, counted = true;
         cnode = rs + min(c, e.x >> 29);
         if (NS > 1 && real) {
@@ -632,7 +634,7 @@ __global__ void __launch_bounds__(kWalkThreads, walk_resident<LPP, COMP>()) walk
         float4 q = __ldg(&a.cm[cnode]);
         const uint4 w = __ldg(reinterpret_cast<const uint4*>(a.info) + cnode);  // WalkInfo
         cchild = w.y;
-        ccnt = w.z & ~kLeafBit;
+        ccnt = real ? w.z & ~kLeafBit : 0u;
         csize = __uint_as_float(w.w);
         const bool heavy = real && q.w != 0.0f;
         isleaf = real && (w.z & kLeafBit);
@@ -662,11 +664,13 @@ __global__ void __launch_bounds__(kWalkThreads, walk_resident<LPP, COMP>()) walk
       __syncwarp();
       // eps^2 per range; a lane inactive for a range adds +inf: it accepts every child, and
       // adds nothing as rsqrt gives 0, and so it sets no open bit (nor does a slot past a
-      // range's count, a dummy with the threshold -inf)
+      // range's count, a dummy with the threshold -inf). A NaN distance (the lane's own position
+      // or a centre of mass) or threshold fails the compare and does set one, in ranges the
+      // lane is inactive for and at dummies too: these are dropped below
       float e2[kWalkRanges];
 #pragma unroll
       for (int r = 0; r < kWalkRanges; r++) e2[r] = masks[r] & lanebit ? eps2 : INFINITY;
-      uint32_t obits = 0;  // children this lane opens (active, not accepted), bit = slot
+      uint32_t obits = 0;  // children this lane does not accept, bit = slot
       // COMP: the round's far-field terms (at most 32 per lane) are summed plainly,
       // then the round's sum joins the particle's total in one Kahan step
       float2 rax = f2(0.f), ray = f2(0.f), raz = f2(0.f), rpt = f2(0.f);
@@ -713,7 +717,6 @@ __global__ void __launch_bounds__(kWalkThreads, walk_resident<LPP, COMP>()) walk
         kahan_add2(F.az, caz, raz);
         kahan_add2(F.pt, cpt, rpt);
       }
-      const uint32_t om = __reduce_or_sync(full, obits);  // children opened by some lane
       if (DBG) {
         uint32_t keep = 0;  // the slots this lane tests, of the ranges it is active for
 #pragma unroll
@@ -733,29 +736,30 @@ __global__ void __launch_bounds__(kWalkThreads, walk_resident<LPP, COMP>()) walk
           if (((obits & ~skipm) >> cc) & 1u) selfw += 1.0f;
         }
       }
-      if (!om) continue;
+      if (!__any_sync(full, obits != 0u)) continue;
       // Every slot's open mask at once: lane c's col holds the lanes that open
       // slot c (the transpose of the 32 x 32 bit matrix whose rows are the lanes'
       // obits), so each slot's lane can act on its own child in parallel. Only
       // the share that tests slot c has its bits: shifted down, they are the
-      // item's particle mask.
-      const uint32_t col = (warp_transpose(obits, lane) >> ((((uint32_t)lane >> 1) % LPP) * G)) & GMASK;
+      // item's particle mask, of which those that opened the slot's parent count.
+      const uint32_t col = (warp_transpose(obits, lane) >> ((((uint32_t)lane >> 1) % LPP) * G)) & act;
+      const uint32_t om = __ballot_sync(full, col != 0u);  // children opened by some particle
       // opened internal children: each slot's lane writes its child range and open
       // mask to the stack, in slot order (prefix positions)
-      const uint32_t pushc = om & ~leafmask;
-      if (pushc) {
-        const int np = __popc(pushc);
+      if (om & ~leafmask) {
+        // a galaxy's child ranges stay in its node range by construction (build,
+        // upload check); the walk itself only guards the pool bounds. A refused range
+        // (a dummy has no children) stays off the stack.
+        const bool push = col != 0u && !isleaf;
+        const bool ok = push && cchild > cnode && ccnt - 1u < 8u && cchild <= a.node_pool - ccnt;
+        if (push && !ok) raise_err(sst, GS_DERR_TREE);
+        const uint32_t okm = __ballot_sync(full, ok);
+        const int np = __popc(okm);
         if (sp + np > kWalkStack) {  // not for depth <= 10 trees
           if (lane == 0) raise_err(sst, GS_DERR_STACK);
         } else {
-          if ((pushc >> lane) & 1u) {
-            // a galaxy's child ranges stay in its node range by construction (build,
-            // upload check); the walk itself only guards the pool bounds
-            const bool ok = cchild > cnode && ccnt - 1u < 8u && cchild <= a.node_pool - ccnt;
-            if (!ok) raise_err(sst, GS_DERR_TREE);
-            S.stack[kWalkRanges + sp + __popc(pushc & below)] =
-                ok ? make_uint2(cchild | ((ccnt - 1u) << 29), col) : make_uint2(0u, 0u);
-          }
+          if (ok)
+            S.stack[kWalkRanges + sp + __popc(okm & below)] = make_uint2(cchild | ((ccnt - 1u) << 29), col);
           sp += np;
         }
       }
