@@ -730,7 +730,8 @@ __global__ void __launch_bounds__(kWalkThreads, walk_resident<LPP, COMP>()) walk
         const uint32_t cc = __ffs(bb) - 1;
         const uint32_t lf = __shfl_sync(full, cchild, cc), cnt = __shfl_sync(full, ccnt, cc);
         const float sz = __shfl_sync(full, csize, cc);
-        if ((top[-(int)(cc >> 3)].y & lanebit) && (i - lf) < cnt) {
+        // the slot's own mask: the stack entry it came from is overwritten by this round's pushes
+        if ((__shfl_sync(full, act, cc) & lanebit) && (i - lf) < cnt) {
           dens = (float)cnt / (sz * sz * sz);
           // the leaf's direct sum includes the particle itself (softened walks)
           if (((obits & ~skipm) >> cc) & 1u) selfw += 1.0f;
