@@ -347,9 +347,11 @@ __device__ __forceinline__ void leaf_flush(Smem& S, const float4* __restrict__ p
           if (m) S.list[n + __popc(b & below)] = (16 * (lane + 32 * r)) | (m << 24);
           n += __popc(b);
         }
+        // no pair of this subgroup's: leave before the padding, which the next subgroup's list
+        // would overwrite with no ordering of the two
+        if (n == 0) continue;
         if (lane < (int)SH) S.list[n + lane] = 0u;
       }
-      if (NSUB > 1 && n == 0) continue;  // no pair of this subgroup's
       __syncwarp();
       const float2 px = f2(NSUB > 1 ? __shfl_sync(full, nx, SUBT * g + tl) : nx);
       const float2 py = f2(NSUB > 1 ? __shfl_sync(full, ny, SUBT * g + tl) : ny);
