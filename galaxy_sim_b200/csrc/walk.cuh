@@ -429,10 +429,12 @@ __device__ inline uint32_t set_gt_mask(float a, float b) {
   return r;
 }
 
-// The largest finite x >= 0 for which theta2 * x > s2 does not hold in FP32 (the product
-// grows with x): x > open_threshold(s2, theta2) decides like theta2 * x > s2 for every x
-// but infinity with theta2 = 0. Searched on the bits, from around s2 / theta2.
+// The largest x >= 0, infinity included, for which theta2 * x > s2 does not hold in FP32 (the
+// product grows with x): x > open_threshold(s2, theta2) decides like theta2 * x > s2 for every x.
+// It is infinity where nothing is accepted: a size beyond 1.8e19 (its square overflows), theta2 = 0.
+// Otherwise searched on the bits, from around s2 / theta2.
 __device__ __noinline__ float open_threshold(float s2, float theta2) {
+  if (!(theta2 * INFINITY > s2)) return INFINITY;
   uint32_t lo = 0u, hi = 0x7f7fffffu;  // holds not at lo
   if (!(theta2 * __uint_as_float(hi) > s2)) return __uint_as_float(hi);
   const uint32_t q = __float_as_uint(s2 / theta2);
@@ -505,16 +507,18 @@ __global__ void __launch_bounds__(kWalkThreads, walk_resident<LPP, COMP>()) walk
   // are size^2's plus one number for all of them; other sizes (uploaded trees) are
   // searched for. It saves a packed multiply per pair; a warp of smaller groups walks too
   // few pairs to earn back the set-up (walk of 524288 particles 972 -> 951 us; of 60001, in
-  // groups of 16, 99 -> 101) and multiplies by theta^2, kept above zero so that an inactive lane's
-  // infinite distance is always far.
+  // groups of 16, 99 -> 101) and multiplies by theta^2. Where theta^2 is zero (or NaN) nothing is
+  // accepted: the multiplier is then the smallest normal float, so that an inactive lane's infinite
+  // distance and a dummy are far as ever, and thr_zero makes every other threshold infinite.
   constexpr bool kThr = LPP == 1;
-  float theta2;
+  float theta2, thr_zero = 0.f;
   uint32_t root_s2 = 0, thr_add = 0, thr_range = 0, thr_slot = 0xffffffffu;
   auto threshold_of = [&](const SegDesc& g) {
     const float theta = __ldg(&a.st[g.slot].p.theta);
     theta2 = theta * theta;
     if (!kThr) {
-      theta2 = fmaxf(theta2, 1.17549435e-38f);
+      thr_zero = theta2 > 0.f ? 0.f : INFINITY;
+      if (!(theta2 > 0.f)) theta2 = 1.17549435e-38f;
       return;
     }
     root_s2 = __float_as_uint(a.info[g.node_off].s2);
@@ -648,7 +652,7 @@ __global__ void __launch_bounds__(kWalkThreads, walk_resident<LPP, COMP>()) walk
         // massless), and sub-softening children
         float thr = -INFINITY;
         if (heavy && !(s2 < qe2)) {
-          thr = kThr ? __uint_as_float(w.x + thr_add) : s2;
+          thr = kThr ? __uint_as_float(w.x + thr_add) : s2 + thr_zero;
           if (kThr && (((w.x ^ root_s2) & 0x7fffffu) || w.x - 0x10000000u >= thr_range)) thr = open_threshold(s2, theta2);
         }
         if (!heavy) q = make_float4(1e30f, 1e30f, 1e30f, 0.f);

@@ -105,3 +105,48 @@ def test_a_lost_galaxy_leaves_its_pool_alone(gpu_lib, kind):
         assert pool.device_errors(slots[k]) == 0
         sim.destroy()
     pool.close()
+
+
+@pytest.mark.parametrize("group,split", SETTINGS)
+@pytest.mark.parametrize("per", [12, 50])
+def test_sizes_whose_squares_overflow(gpu_lib, oracle, per, group, split):
+    """Two clumps 2e20 apart: size^2 of the upper nodes and r^2 between the clumps are +inf,
+    such a node is never accepted, and the particles of a clump attract one another. The
+    other clump's pull is 1e-18 of that and 0 in FP32; the rest are a few dozen terms
+    summed in FP32."""
+    P0 = np.zeros((2 * per, 8), np.float32)
+    P0[:, 0] = np.repeat([-1e20, 1e20], per)
+    P0[:, 1] = np.tile(np.arange(per) * 1e10, 2)
+    P0[:, 3] = 1.0
+    sim = NBodyGPU(0, P0, walkGroup=group, walkSplit=split)
+    sim.updateParams(dt=0.0, G=1.0, epsilon=0.0, theta=0.5)
+    sim.setDebug(True)
+    sim.sortBuild()
+    P, _ = sim.readState()
+    nodes, lr, _ = sim.getTree()
+    sim.step()
+    assert sim.deviceErrors() == 0
+    acc, _ = sim.readForces()
+    sim.destroy()
+    p = oracle.make_params(2 * per, epsilon=0.0, theta=0.5, dt=0.0)
+    want, _, _, _ = oracle.walk_f64(p, P, nodes, oracle.refresh_f64(P, nodes, lr))
+    assert np.all(np.abs(acc[:, 1] - want[:, 1]) <= 1e-5 * np.abs(want[:, 1]).max())
+    assert np.abs(want[:, 1]).max() > 1e-20
+
+
+@pytest.mark.parametrize("group,split", SETTINGS)
+@pytest.mark.parametrize("n,far", [(5, None), (700, None), (700, 1e5), (700, 3e19)])
+def test_zero_opening_angle_opens_every_node(gpu_lib, n, far, group, split):
+    P0 = ic.hernquist_sphere(n, 90 + n).particles.copy()
+    if far:
+        P0[n // 3, 0] = far
+    sim = NBodyGPU(0, P0, walkGroup=group, walkSplit=split)
+    sim.updateParams(dt=0.0, G=1.0, epsilon=1e-3, theta=0.0)
+    sim.setDebug(True)
+    sim.sortBuild()
+    nodes, _, _ = sim.getTree()
+    sim.counters(reset=True)
+    sim.step()
+    assert sim.counters() == [0, n * (n - 1), n * len(nodes)]
+    assert sim.deviceErrors() == 0
+    sim.destroy()
