@@ -259,10 +259,31 @@ __global__ void __launch_bounds__(kFlagThreads)
       }
       uint32_t end = base + hi;
       if (c0 + tid + 1 == nstart && dnext > (uint32_t)L) {  // it goes on in the next tile
-        for (; end < seg_end; end++) {
-          const uint32_t x = b.dl[end];
-          if ((x & 15u) <= x >> 4) break;
-          sum.add(pos[2 * (size_t)end]);
+        // its end first, past tiles without a start by their counts, then by the flags, then its
+        // records, both kComChunk loads at a time: one particle per trip, its flag before its
+        // record, took 11.2 ms for the rebuild of 100000 particles half of which are at one
+        // place, 2.6 ms so (sphere of 200003: 88 -> 86 us)
+        const uint32_t from = end;
+        for (uint32_t x = tile + 1; end < seg_end && b.blk_counts[(size_t)x * kTileWords + kMaxLevel + 1] == 0; x++)
+          end += P;
+        for (bool more = end < seg_end; more; more = more && end < seg_end) {
+          uint32_t f[kComChunk];
+#pragma unroll
+          for (uint32_t k = 0; k < kComChunk; k++) f[k] = end + k < seg_end ? b.dl[end + k] : 0u;
+#pragma unroll
+          for (uint32_t k = 0; k < kComChunk; k++) {
+            more = more && (f[k] & 15u) > f[k] >> 4;  // past the galaxy: 0, a start
+            end += more ? 1u : 0u;
+          }
+        }
+        end = min(end, seg_end);
+        for (uint32_t k0 = from; k0 < end; k0 += kComChunk) {
+          float4 q[kComChunk];
+#pragma unroll
+          for (uint32_t k = 0; k < kComChunk; k++) q[k] = pos[2 * (size_t)min(k0 + k, end - 1)];
+#pragma unroll
+          for (uint32_t k = 0; k < kComChunk; k++)
+            if (k0 + k < end) sum.add(q[k]);
         }
       }
       const float4 c = sum.mean();
