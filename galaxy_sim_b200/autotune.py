@@ -14,11 +14,12 @@ Knobs (`gs_set_tuning`):
   Like the group size it changes only the order of the force sums. A pool of
   several galaxies walks unsplit, so the tuner skips this knob there;
 * the persistent walk grid (blocks per SM; groups are independent, so fewer
-  resident warps only change the schedule; below 8 the walk compiled for 72
-  registers per thread runs) - never changes results;
+  resident warps only change the schedule; at most 7 are launched, so a setting
+  of 8 runs the same grid as 7 and is no candidate) - never changes results;
 * the sort tile depth (4, 8 or 16 keys per thread: tiles of 1024, 2048 or 4096
   keys; a small galaxy sorts in more tiles with the smaller depths; a stable
-  sort has one answer) - never changes results.
+  sort has one answer) - never changes results. A lone galaxy that is rebuilt by
+  one kernel has no sort tiles: one depth is timed there.
 
 The bucket size (16) is not a knob: it is the reference's tree
 (mortonTree.js:25), and changing it would change every result.
@@ -38,7 +39,7 @@ import itertools
 from ._lib import (TUNE_SORT_ITEMS, TUNE_WALK_BLOCKS_PER_SM, TUNE_WALK_GROUP, TUNE_WALK_SPLIT, GalaxyError,
                    check, lib)
 
-WALK_BLOCKS = (6, 7, 8)
+WALK_BLOCKS = (6, 7)
 SORT_ITEMS = (4, 8, 16)
 WALK_GROUPS = (0, 4, 8, 16, 32)
 WALK_SPLITS = (0, 1, 2, 4, 8)
@@ -60,6 +61,13 @@ def launch_setting(ctx) -> dict:
     g, s, i = C.c_uint32(0), C.c_uint32(0), C.c_uint32(0)
     check(lib().gs_get_launch_setting(ctx, C.byref(g), C.byref(s), C.byref(i)), ctx)
     return {"walk_group": g.value, "walk_split": s.value, "sort_keys_per_thread": i.value}
+
+
+def _one_kernel_rebuild(ctx) -> bool:
+    """Whether the last captured step was rebuild, walk and diagnostics, a kernel each."""
+    n = C.c_uint32(0)
+    check(lib().gs_step_kernels(ctx, C.byref(n)), ctx)
+    return n.value == 3
 
 
 def _time(owner, ext, steps, warmup, star_formation):
@@ -101,6 +109,10 @@ def autotune(owner, steps: int = 5, warmup: int = 2, star_formation: bool = Fals
         set_(ctx, TUNE_WALK_SPLIT, best_split)
     else:
         best_split = get(ctx, TUNE_WALK_SPLIT)
+    sort_items = tuple(sort_items)
+    if lone and _one_kernel_rebuild(ctx):                 # the sort has no tiles
+        cur = get(ctx, TUNE_SORT_ITEMS)
+        sort_items = (cur if cur in sort_items else sort_items[0],)
     timing = {}
     for bps, items in itertools.product(walk_blocks, sort_items):
         try:

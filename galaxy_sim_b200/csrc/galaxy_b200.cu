@@ -718,11 +718,15 @@ void enqueue_build(gs_ctx* c, const float4* pos, uint32_t stride, double root_si
   launch_pdl(tree_leaves_kernel<kComJs>, L.flag_tiles, kLeafThreads, s, b, L, pos, stride, c->st);
 }
 
+// g blocks, at most those that are resident at once (persistent warps take all the items)
 template <int LPP>
-void launch_walk(int v, uint32_t g, cudaStream_t s, const WalkArgs& a) {
+void launch_walk(int v, uint32_t g, uint32_t sms, cudaStream_t s, const WalkArgs& a) {
   switch (v) {
 #define GS_WALK_CASE(V, SF, DBG, ONE, COMP) \
-  case V: launch_pdl(walk_kernel<SF, DBG, ONE, COMP, LPP>, g, kWalkThreads, s, a); break;
+  case V:                                                                                                  \
+    launch_pdl(walk_kernel<SF, DBG, ONE, COMP, LPP>, std::min<uint32_t>(g, sms * walk_resident<LPP, COMP>()), \
+               kWalkThreads, s, a);                                                                        \
+    break;
     GS_WALK_CASE(0, false, false, false, false)
     GS_WALK_CASE(1, true, false, false, false)
     GS_WALK_CASE(2, false, true, false, false)
@@ -773,10 +777,10 @@ void enqueue_walk(gs_ctx* c, int sf) {
   for (int k = 0; k < 4; k++) {
     if (!c->walk_items[k]) continue;
     const uint32_t gk = std::min<uint32_t>(g, std::max<uint32_t>(1, cdiv(c->walk_items[k], kWalkWarps)));
-    if (k == 0) launch_walk<1>(v, gk, s, a);
-    else if (k == 1) launch_walk<2>(v, gk, s, a);
-    else if (k == 2) launch_walk<4>(v, gk, s, a);
-    else launch_walk<8>(v, gk, s, a);
+    if (k == 0) launch_walk<1>(v, gk, c->sms, s, a);
+    else if (k == 1) launch_walk<2>(v, gk, c->sms, s, a);
+    else if (k == 2) launch_walk<4>(v, gk, c->sms, s, a);
+    else launch_walk<8>(v, gk, c->sms, s, a);
   }
   // per-galaxy FP64 diagnostics of this walk
   launch_pdl(diag_reduce_kernel, c->lay.diag_chunks, 32 * kPartials, s, (const double*)c->partials, c->lay,

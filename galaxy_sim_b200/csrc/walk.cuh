@@ -61,11 +61,11 @@ constexpr int kWalkStack = 8 * 11 * kWalkRanges;
 // KB of staging per block let onto an SM, at 72 registers per thread (6 at 80 registers:
 // walk of 524288 particles 953 -> 968 us; compensated sums need the 80: 306 -> 290 us on a
 // sphere of 200003). Smaller groups walk small galaxies, which do not fill the SMs, and
-// run without spills and with more loads in flight at more registers: full step at 7 / 6
+// run with fewer spills and more loads in flight at more registers: full step at 7 / 6
 // / 5 blocks in us: 4096 particles 62.1 / 61.2 / 60.0, 16384 106.0 / 101.1 / 101.8, 25000 133 / 131 / 124
 // (groups of 8); 60001 163 / 157 / 164, 100000 310 / 308 / 303 (groups of 16). The launch
-// tuning accepts 1..8 blocks per SM; more than the resident ones launch no further ones.
-constexpr int kWalkBlocksPerSM = 8;
+// tuning accepts 1..8 blocks per SM; no more are launched than the resident ones.
+constexpr int kWalkBlocksPerSM = 8;  // the tuning's largest value
 constexpr int kWalkResident = 7;
 template <int LPP, bool COMP>
 constexpr int walk_resident() {

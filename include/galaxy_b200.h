@@ -123,8 +123,9 @@ int gs_set_walk_mode(gs_ctx* ctx, int compensated);
 /* Launch tuning (no counterpart in the reference). Takes effect at the next step;
  * galaxy_sim_b200/autotune.py picks values by timing.
  * GS_TUNE_WALK_BLOCKS_PER_SM = persistent walk blocks per SM (1..8; default 7 for a
- * gs_create context, 8 for a pool; 7 blocks fit an SM, so 8 runs 7); never
- * changes results.
+ * gs_create context, 8 for a pool; no more are launched than fit an SM: 7 for walk
+ * groups of 32, 6 for groups of 16 and with compensated sums, 5 for groups of 8 and 4);
+ * never changes results.
  * GS_TUNE_SORT_ITEMS = keys per thread of a sort tile (4, 8 or 16, or 0 = by the
  * largest galaxy's size: 4 up to 131072 particles, 8 up to 393216, else 16;
  * default 0 for a gs_create context, 16 for a pool; a lone galaxy of at most 32768
