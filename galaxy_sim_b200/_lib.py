@@ -71,6 +71,7 @@ SIGNATURES = [
     ("gs_apply_permutation", _int, [_vp, _vp]),
     ("gs_upload_tree", _int, [_vp, _vp, _u32, _vp, _u32]),
     ("gs_refresh", _int, [_vp]),
+    ("gs_refresh_kernels", _int, [_vp, _vp]),
     ("gs_step", _int, [_vp]),
     ("gs_star_formation", _int, [_vp]),
     ("gs_read_positions", _int, [_vp, _vp, C.c_uint64]),

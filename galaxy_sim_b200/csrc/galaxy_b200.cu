@@ -265,6 +265,7 @@ struct gs_ctx {
   bool rb_pending = false;
   std::map<int, cudaGraphExec_t> graphs;
   uint32_t step_kernels = 0;  // kernel nodes of the last captured step graph
+  uint32_t refresh_kernels = 0;  // kernels the last gs_refresh launched
   char err[512] = "";
 
   int fail(int code, const char* fmt, ...) {
@@ -1315,6 +1316,7 @@ int gs_refresh(gs_ctx* ctx) {
   int rc = ensure_layout(ctx);
   if (rc) return rc;
   bool built = false;
+  ctx->refresh_kernels = 0;
   for (Slot& s : ctx->slots) {
     if (!s.live) continue;
     if (s.tree == Slot::kTreeBuilt) built = true;
@@ -1347,16 +1349,19 @@ int gs_refresh(gs_ctx* ctx) {
       cudaLaunchAttribute attr[2];
       refresh_config(cfg, attr, ctx->stream);
       cudaLaunchKernelEx(&cfg, refresh_internal_kernel, ctx->cm, (const WalkInfo*)ctx->info, lv);
+      ctx->refresh_kernels += 2;
       continue;
     }
     for (int64_t l = nl - 1; l >= 0; l--) {
       const uint32_t start = s.up_lr[2 * l], count = s.up_lr[2 * l + 1];
-      if (count)
-        refresh_level_kernel<<<cdiv(count, 64), 64, 0, ctx->stream>>>(ctx->part[ctx->cur], ctx->cm, ctx->info,
-                                                                       s.node_off + start, count);
+      if (!count) continue;
+      refresh_level_kernel<<<cdiv(count, 64), 64, 0, ctx->stream>>>(ctx->part[ctx->cur], ctx->cm, ctx->info,
+                                                                     s.node_off + start, count);
+      ctx->refresh_kernels++;
     }
   }
   if (built && ctx->lay.nseg) {
+    ctx->refresh_kernels++;
     BuildBuffers b = ctx->bb();
     const Layout& L = ctx->lay;
     if (ctx->com_mode == kComF64)
@@ -1649,6 +1654,13 @@ int gs_step_kernels(gs_ctx* ctx, uint32_t* n) {
   CTX_CHECK(ctx);
   if (!n) return ctx->fail(GS_EINVAL, "n is NULL");
   *n = ctx->step_kernels;
+  return GS_OK;
+}
+
+int gs_refresh_kernels(gs_ctx* ctx, uint32_t* n) {
+  CTX_CHECK(ctx);
+  if (!n) return ctx->fail(GS_EINVAL, "n is NULL");
+  *n = ctx->refresh_kernels;
   return GS_OK;
 }
 

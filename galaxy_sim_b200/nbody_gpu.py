@@ -223,6 +223,12 @@ class NBodyGPU:
         self._ok(lib().gs_step_kernels(self._ctx, C.byref(n)))
         return n.value
 
+    def refreshKernels(self) -> int:
+        """Kernel launches of the last encodeRefresh."""
+        n = C.c_uint32(0)
+        self._ok(lib().gs_refresh_kernels(self._ctx, C.byref(n)))
+        return n.value
+
     @property
     def stream(self) -> int:
         d = C.c_void_p()

@@ -171,6 +171,10 @@ int gs_upload_tree(gs_ctx* ctx, const gs_node* nodes, uint32_t num_nodes,
                    const uint32_t* level_ranges, uint32_t n_levels);
 /* NBodyGPU.encodeRefresh (NBodyGPU.js:308-319) → refresh_level deepest first. */
 int gs_refresh(gs_ctx* ctx);
+/* Kernel launches of the last gs_refresh (0 before the first): two for an uploaded tree
+ * whose level ranges follow one another, else one per level that has nodes; one more
+ * for all galaxies whose trees were built on the device. */
+int gs_refresh_kernels(gs_ctx* ctx, uint32_t* n);
 /* NBodyGPU.step (NBodyGPU.js:321-329): walk + halo + kick-drift, flip. */
 int gs_step(gs_ctx* ctx);
 /* NBodyGPU.encodeStarFormation (NBodyGPU.js:278-285). */
