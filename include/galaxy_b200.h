@@ -47,7 +47,8 @@ extern "C" {
 #define GS_DERR_LOOKBACK 0x1u   /* sort look-back wait exceeded its iteration limit */
 #define GS_DERR_STACK 0x2u      /* walk stack deeper than the tree can be */
 #define GS_DERR_NODES 0x4u      /* node pool exhausted */
-#define GS_DERR_TREE 0x8u       /* uploaded tree is not a BFS tree with contiguous children */
+#define GS_DERR_TREE 0x8u       /* uploaded tree is not a BFS tree with contiguous children, or a
+                                 * particle at a NaN position walked (its galaxy steps on) */
 
 typedef struct gs_ctx gs_ctx;
 
