@@ -150,3 +150,31 @@ def test_zero_opening_angle_opens_every_node(gpu_lib, n, far, group, split):
     assert sim.counters() == [0, n * (n - 1), n * len(nodes)]
     assert sim.deviceErrors() == 0
     sim.destroy()
+
+
+@pytest.mark.parametrize("n", [300, 5000, 40000])
+@pytest.mark.parametrize("kind", ["one", "inf", "all"])
+def test_steps_equal_a_pools(gpu_lib, n, kind):
+    """Full steps of such a galaxy alone (one rebuild kernel up to 32768 particles) and
+    in a pool (separate rebuild kernels): the same finite values, NaNs at the same places,
+    the same error word."""
+    g = ic.hernquist_sphere(n, 60 + n)
+    P0 = g.particles.copy()
+    if kind == "all":
+        P0[:, :3] = np.nan
+    else:
+        P0[n // 2, 0] = np.nan if kind == "one" else np.inf
+    other = ic.hernquist_sphere(100, 7)
+    sim = NBodyGPU(0, P0, g.stellar, walkGroup=32, walkSplit=1)
+    pool = GalaxyPool(-(-n // 256) * 256 + 256, 2)
+    slot, fine = pool.add(P0, g.stellar, KW), pool.add(other.particles, other.stellar, KW)
+    sim.updateParams(**KW)
+    sim.run(2, False)
+    pool.run(2, False)
+    err = sim.deviceErrors(clear=True)
+    assert err == pool.device_errors(slot, clear=True) and pool.device_errors(fine) == 0
+    for a, b in zip(sim.readState(), pool.read_state(slot)):
+        assert np.array_equal(a, b, equal_nan=True)
+    assert (sim.stepKernels() == 3) == (n <= 32768)
+    sim.destroy()
+    pool.close()
